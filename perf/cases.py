@@ -5,9 +5,10 @@ A case is a model (the widths of the presets, fewer layers where layers repeat),
   call "generate"  Engine.generate: every row decodes `new` tokens behind its prompt, one captured step per token.  run() is
                    the retry of a call that prepare() made: agents resubmit identical prompts up to two times, so a dense
                    model finds the prompts' pages in its prefix cache and computes the part of a page that is left; layer
-                   stacks keep no prefix and compute the prompts again.  Rows decode under the game's vote grammar and are
-                   forced through "{" and blanks, which it allows without end, so that every pass runs every row to the end
-                   over the same tokens whatever its random logits favour.
+                   stacks keep no prefix and compute the prompts again.  Rows are forced through given tokens, so that every
+                   pass runs every row to the end over the same tokens whatever its random logits favour: a dense model's under
+                   the game's vote grammar through "{" and blanks, which it allows without end, a stack's through tokens of
+                   their own (rows choose experts of their own).
   call "replay"    Engine.open / step / close_sequence: `join` sequences are admitted per step (0: all at once), prompts
                    come in portions of at most `portion` tokens (0: whole) beside the single tokens of the sequences that
                    are through, `new` of them each.  Logits are wanted behind the
@@ -242,18 +243,13 @@ def _tensors(cfg, seed):
     return out
 
 
-def _tokens(case, cfg, seed, feed):
-    """Every row's tokens: a prompt and what is fed behind it."""
-    rng = np.random.default_rng(seed)
-    return [rng.integers(0, cfg.vocab, n).tolist() + (feed if feed else rng.integers(0, cfg.vocab, case["new"]).tolist())
-            for n in _lengths(case)]
-
-
-def _feed(case, cfg):
-    if case["call"] == "replay":
-        return []
-    tk = get_tokenizer("qwen3", cfg.vocab)
-    return tk.encode("{", False) + tk.encode(" ", False) * (case["new"] - 1)
+def _tokens(case, cfg, seed):
+    """Every row's tokens: a prompt and what is fed behind it (no stop tokens, which are the last ones)."""
+    rng, feed = np.random.default_rng(seed), []
+    if case["call"] == "generate" and case["model"] not in STACKS:
+        tk = get_tokenizer("qwen3", cfg.vocab)
+        feed = tk.encode("{", False) + tk.encode(" ", False) * (case["new"] - 1)
+    return [rng.integers(0, cfg.vocab, n).tolist() + (feed or rng.integers(0, cfg.vocab // 2, case["new"]).tolist()) for n in _lengths(case)]
 
 
 def prepare(case, seed):
@@ -272,11 +268,11 @@ def prepare(case, seed):
         launch = sum(lens)
     engine = Engine(cfg, w, get_tokenizer("qwen3", cfg.vocab) if generate else None, max_model_len=blocks * PAGE, max_rows=case["rows"],
                     prefill_tokens=min(16384, -(-launch // 128) * 128), kv_pages=case["rows"] * blocks + 8, logit_rows=128 if case["want"] > 1 else 0)
-    fed = _feed(case, cfg)
-    tokens = _tokens(case, cfg, seed, fed)
+    tokens = _tokens(case, cfg, seed)
     state = dict(engine=engine, rows=case["rows"], vocab=cfg.vocab)
     if generate:
-        state["requests"] = [Request("", VOTE, 0.3, case["new"], forced=fed, prompt_ids=t[:n]) for t, n in zip(tokens, lens)]
+        schema = None if case["model"] in STACKS else VOTE
+        state["requests"] = [Request("", schema, 0.3, case["new"], forced=t[n:], prompt_ids=t[:n]) for t, n in zip(tokens, lens)]
         engine.generate(state["requests"])
     else:
         state["steps"] = [[(r, tokens[r][a:a + n], list(range(n - want, n))) for r, a, n, want in step] for step in _schedule(case)]
@@ -542,7 +538,7 @@ def _stack(cfg, w, x, pos):
 def exact(case, seed):
     cfg = _config(case)
     w = _tensors(cfg, seed)
-    tokens = _tokens(case, cfg, seed, _feed(case, cfg))
+    tokens = _tokens(case, cfg, seed)
     n = max(len(t) for t in tokens)
     ids = torch.tensor([t + [0] * (n - len(t)) for t in tokens], device="cuda")
     pos = torch.arange(n, device="cuda")
