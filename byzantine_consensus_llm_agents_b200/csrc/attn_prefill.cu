@@ -133,7 +133,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {      // one elected thread per role: see gemm_tcgen05.cu
       pdl_wait();   // q and this step's KV rows come from the kernels in front of this one
       mbar_arrive_expect_tx(q_full, kPfQTile);
       tma_load_2d(smem + C::kOffQ, &q_map, q_full, head * 128, row0, kEvictFirst);
@@ -168,52 +168,47 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    const uint32_t sq = smem_u32(smem + C::kOffQ);
-    const uint32_t sp = smem_u32(smem + C::kOffP);
+    // descriptors' address fields count 16 bytes; all tiles lie below 256 KB, so that offsets add up without a carry
+    const uint64_t desc_q = make_kmajor_sw128_desc(smem_u32(smem + C::kOffQ));
+    const uint64_t desc_p = make_kmajor_sw128_desc(smem_u32(smem + C::kOffP));
+    const uint64_t desc_k = make_kmajor_sw128_desc(smem_u32(smem + C::kOffK));
+    const uint64_t desc_v = make_mnmajor_sw128_desc(smem_u32(smem + C::kOffV), C::kKvHalf);
     auto issue_s = [&](int j) {
       const int st = j & 1;
       const uint32_t par = (j >> 1) & 1;
       mbar_wait(&k_full[st], par);
       mbar_wait(&s_free[st], par ^ 1);
       tc_fence_after();
-      if (lane == 0) {
-        const uint32_t sk = smem_u32(smem + C::kOffK + st * C::kKvTile);
-        const uint32_t d = tmem_base + static_cast<uint32_t>(st * BN);
+      const uint64_t dk = desc_k + static_cast<uint64_t>(st * (C::kKvTile >> 4));
+      const uint32_t d = tmem_base + static_cast<uint32_t>(st * BN);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {   // head_dim 128 = 8 x k16; halves of 64, 32 B per step
-          umma_bf16(d, make_kmajor_sw128_desc(sq + (ks >> 2) * kPfQHalf + (ks & 3) * 32),
-                    make_kmajor_sw128_desc(sk + (ks >> 2) * C::kKvHalf + (ks & 3) * 32), kIdescQK,
-                    ks > 0 ? 1u : 0u);
-        }
-        umma_commit(&k_empty[st]);
-        umma_commit(&s_full[st]);
-      }
-      __syncwarp();
+      for (int ks = 0; ks < 8; ++ks)   // head_dim 128 = 8 x k16; halves of 64, 32 B per step
+        umma_bf16(d, desc_q + (((ks >> 2) * kPfQHalf + (ks & 3) * 32) >> 4), dk + (((ks >> 2) * C::kKvHalf + (ks & 3) * 32) >> 4),
+                  kIdescQK, ks > 0 ? 1u : 0u);
+      umma_commit(&k_empty[st]);
+      umma_commit(&s_full[st]);
     };
     auto issue_pv = [&](int j) {
       const int st = j & 1;
       mbar_wait(p_full, j & 1);          // P_j written (and O rescaled where that was needed)
       mbar_wait(&v_full[st], (j >> 1) & 1);
       tc_fence_after();
-      if (lane == 0) {
-        const uint32_t sv = smem_u32(smem + C::kOffV + st * C::kKvTile);
+      const uint64_t dv = desc_v + static_cast<uint64_t>(st * (C::kKvTile >> 4));
 #pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk) {
-          // P: K-major, 64-token halves of 16 KB, 32 B per k16 step; V: 16 token rows of 128 B per step
-          umma_bf16(tmem_o, make_kmajor_sw128_desc(sp + (kk >> 2) * kPfQHalf + (kk & 3) * 32),
-                    make_mnmajor_sw128_desc(sv + kk * 16 * 128, C::kKvHalf), kIdescPV,
-                    (j > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(&v_empty[st]);
-        umma_commit(pv_done);
-      }
-      __syncwarp();
+      for (int kk = 0; kk < BN / 16; ++kk)
+        // P: K-major, 64-token halves of 16 KB, 32 B per k16 step; V: 16 token rows of 128 B per step
+        umma_bf16(tmem_o, desc_p + (((kk >> 2) * kPfQHalf + (kk & 3) * 32) >> 4), dv + ((kk * 16 * 128) >> 4), kIdescPV,
+                  (j > 0 || kk > 0) ? 1u : 0u);
+      umma_commit(&v_empty[st]);
+      umma_commit(pv_done);
     };
-    mbar_wait(q_full, 0);
-    issue_s(0);
-    for (int j = 0; j < nb; ++j) {
-      if (j + 1 < nb) issue_s(j + 1);
-      issue_pv(j);
+    if (elect_one()) {
+      mbar_wait(q_full, 0);
+      issue_s(0);
+      for (int j = 0; j < nb; ++j) {
+        if (j + 1 < nb) issue_s(j + 1);
+        issue_pv(j);
+      }
     }
   } else {
     // ------------------------------ softmax + output --------------------------

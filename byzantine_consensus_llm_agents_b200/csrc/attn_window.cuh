@@ -183,7 +183,7 @@ window_attn_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const uint32_t tmem_o = tmem_base + 2 * kWaBN;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {      // one elected thread per role: see gemm_tcgen05.cu
       mbar_arrive_expect_tx(q_full, C::kQ);
 #pragma unroll
       for (int c = 0; c < QD / 64; ++c)
@@ -215,46 +215,44 @@ window_attn_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       }
     }
   } else if (warp == 1) {
-    const uint32_t sq = smem_u32(smem);
-    const uint32_t sp = smem_u32(smem + C::kOffP);
+    // descriptors' address fields count 16 bytes; all tiles lie below 256 KB, so that offsets add up without a carry
+    const uint64_t desc_q = make_kmajor_sw128_desc(smem_u32(smem));
+    const uint64_t desc_p = make_kmajor_sw128_desc(smem_u32(smem + C::kOffP));
+    const uint64_t desc_k = make_kmajor_sw128_desc(smem_u32(smem + C::kOffK));
+    const uint64_t desc_v = make_mnmajor_sw128_desc(smem_u32(smem + C::kOffV), kWaKvHalf);
     auto issue_s = [&](int j) {
       const int st = j % ST;
       mbar_wait(&k_full[st], (j / ST) & 1);
       mbar_wait(&s_free[j & 1], ((j >> 1) & 1) ^ 1);
       tc_fence_after();
-      if (lane == 0) {
-        const uint32_t sk = smem_u32(smem + C::kOffK + st * C::kK);
-        const uint32_t d = tmem_base + static_cast<uint32_t>((j & 1) * kWaBN);
+      const uint64_t dk = desc_k + static_cast<uint64_t>(st * (C::kK >> 4));
+      const uint32_t d = tmem_base + static_cast<uint32_t>((j & 1) * kWaBN);
 #pragma unroll
-        for (int ks = 0; ks < QD / 16; ++ks)
-          umma_bf16(d, make_kmajor_sw128_desc(sq + (ks >> 2) * kWaQHalf + (ks & 3) * 32),
-                    make_kmajor_sw128_desc(sk + (ks >> 2) * kWaKvHalf + (ks & 3) * 32), kIdescQK, ks > 0 ? 1u : 0u);
-        umma_commit(&k_empty[st]);
-        umma_commit(&s_full[j & 1]);
-      }
-      __syncwarp();
+      for (int ks = 0; ks < QD / 16; ++ks)
+        umma_bf16(d, desc_q + (((ks >> 2) * kWaQHalf + (ks & 3) * 32) >> 4), dk + (((ks >> 2) * kWaKvHalf + (ks & 3) * 32) >> 4),
+                  kIdescQK, ks > 0 ? 1u : 0u);
+      umma_commit(&k_empty[st]);
+      umma_commit(&s_full[j & 1]);
     };
     auto issue_pv = [&](int j) {
       const int st = j % ST;
       mbar_wait(p_full, j & 1);
       mbar_wait(&v_full[st], (j / ST) & 1);
       tc_fence_after();
-      if (lane == 0) {
-        const uint32_t sv = smem_u32(smem + C::kOffV + st * C::kV);
+      const uint64_t dv = desc_v + static_cast<uint64_t>(st * (C::kV >> 4));
 #pragma unroll
-        for (int kk = 0; kk < kWaBN / 16; ++kk)
-          umma_bf16(tmem_o, make_kmajor_sw128_desc(sp + kk * 32), make_mnmajor_sw128_desc(sv + kk * 16 * 128, kWaKvHalf),
-                    kIdescPV, (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&v_empty[st]);
-        umma_commit(pv_done);
-      }
-      __syncwarp();
+      for (int kk = 0; kk < kWaBN / 16; ++kk)
+        umma_bf16(tmem_o, desc_p + ((kk * 32) >> 4), dv + ((kk * 16 * 128) >> 4), kIdescPV, (j > 0 || kk > 0) ? 1u : 0u);
+      umma_commit(&v_empty[st]);
+      umma_commit(pv_done);
     };
-    mbar_wait(q_full, 0);
-    issue_s(0);
-    for (int j = 0; j < nb; ++j) {
-      if (j + 1 < nb) issue_s(j + 1);
-      issue_pv(j);
+    if (elect_one()) {
+      mbar_wait(q_full, 0);
+      issue_s(0);
+      for (int j = 0; j < nb; ++j) {
+        if (j + 1 < nb) issue_s(j + 1);
+        issue_pv(j);
+      }
     }
   } else {
     const int q4 = warp & 3;

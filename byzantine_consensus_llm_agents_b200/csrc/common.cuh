@@ -104,8 +104,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 // Bounded spin: a protocol bug traps (reported as a CUDA error to the caller)
-// instead of hanging the GPU.
+// instead of hanging the GPU.  The first look stands in front of the counted loop: a barrier that is complete already costs
+// half as much that way (75 instead of 145-180 clocks in the GEMMs' roles, clock64).
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return;
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
     if (++spins > (1u << 26)) __trap();

@@ -176,7 +176,7 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {      // one elected thread per role: see gemm_tcgen05.cu
       pdl_wait();
       int stage = 0;
       uint32_t phase = 0;
@@ -200,7 +200,8 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA) --------------------------------
-    if (leader) {
+    if (leader && elect_one()) {
+      const uint64_t desc0 = make_kmajor_sw128_desc(smem_u32(smem));
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -212,17 +213,13 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         for (int kb = 0; kb < args.k_blocks; ++kb) {
           mbar_wait(&full_bar[stage], phase);
           tc_fence_after();
-          if (lane == 0) {
-            const uint32_t sa = smem_u32(smem + stage * k2StageBytes);
-            const uint64_t da = make_kmajor_sw128_desc(sa);
-            const uint64_t db = make_kmajor_sw128_desc(sa + k2ABytes);
+          const uint64_t da = desc0 + static_cast<uint64_t>(stage * (k2StageBytes >> 4));
+          const uint64_t db = da + (k2ABytes >> 4);
 #pragma unroll
-            for (int k = 0; k < k2BlockK / 16; ++k)
-              umma_bf16_2sm(tmem_d, da + 2 * k, db + 2 * k, k2Idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            umma_commit_2sm(&empty_bar[stage]);
-            if (kb == args.k_blocks - 1) umma_commit_2sm(&tmem_full[acc]);
-          }
-          __syncwarp();
+          for (int k = 0; k < k2BlockK / 16; ++k)
+            umma_bf16_2sm(tmem_d, da + 2 * k, db + 2 * k, k2Idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_2sm(&empty_bar[stage]);
+          if (kb == args.k_blocks - 1) umma_commit_2sm(&tmem_full[acc]);
           if (++stage == k2Stages) {
             stage = 0;
             phase ^= 1;

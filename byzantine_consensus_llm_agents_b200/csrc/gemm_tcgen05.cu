@@ -207,7 +207,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    // One elected thread runs the whole role, here and in the MMA warp: copies and MMAs take their operands from uniform
+    // registers, and behind `lane == 0` the compiler does not know that only one thread is there.  Clocks per 64-wide k-block
+    // that way and this way (one CTA per SM): 16 rows 650 -> 295, tiles of 128 columns 640 -> 295 (the MMAs: 256), of 256
+    // columns 650 -> 538 (512).
+    if (elect_one()) {
       // Under programmatic dependent launch this CTA may start while the previous kernel is still
       // running.  Weights never depend on it, activations do: so the weight halves of the first
       // kPreWaitStages ring slots are requested right away and only then does the producer wait
@@ -263,23 +267,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    int stage = 0;
-    uint32_t phase = 0;
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
-      int ta, tb, split, kb0, kb1, e;
-      decode_item(item, ta, tb, split, kb0, kb1, e);
-      mbar_wait(&tmem_empty[acc], acc_phase ^ 1);
-      tc_fence_after();
-      const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * BN);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        mbar_wait(&full_bar[stage], phase);
+    if (elect_one()) {
+      const uint64_t desc0 = make_kmajor_sw128_desc(smem_u32(smem));   // stage 0, operand A; the address field counts 16 bytes
+      int stage = 0;
+      uint32_t phase = 0;
+      int acc = 0;
+      uint32_t acc_phase = 0;
+      for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+        int ta, tb, split, kb0, kb1, e;
+        decode_item(item, ta, tb, split, kb0, kb1, e);
+        mbar_wait(&tmem_empty[acc], acc_phase ^ 1);
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint64_t da = make_kmajor_sw128_desc(sa);
-          const uint64_t db = make_kmajor_sw128_desc(sa + A_BYTES);
+        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * BN);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          mbar_wait(&full_bar[stage], phase);
+          tc_fence_after();
+          const uint64_t da = desc0 + static_cast<uint64_t>(stage * (STAGE_BYTES >> 4));
+          const uint64_t db = da + (A_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k) {
             // advance 16 bf16 = 32 B inside the 128 B swizzle atom: +2 in the (addr>>4) field
@@ -287,15 +291,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           umma_commit(&empty_bar[stage]);
           if (kb == kb1 - 1) umma_commit(&tmem_full[acc]);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
-        __syncwarp();
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
-        }
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1;
       }
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1;
     }
   } else {
     // ------------------------------ epilogue ----------------------------------
