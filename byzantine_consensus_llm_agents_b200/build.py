@@ -33,6 +33,7 @@ SOURCES = [
     "tp_reduce_norm.cu",
     "stack_norm.cu",
     "gemm_simt.cu",
+    "gemm_split_tcgen05.cu",
     "latent_attn.cu",
     "latent_prefill.cu",
     "grouped_attn.cu",

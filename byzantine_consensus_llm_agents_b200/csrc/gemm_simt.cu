@@ -1,5 +1,6 @@
 // out fp32 [M, ldo] = X [M, ldx] * W bf16 [N, ldw]^T on CUDA cores, fp32 FMA throughout: the product of
-// fp32 activations, and of bf16 ones whose shape TMA cannot address.  64 x 64 tiles, 4 x 4 per thread.
+// fp32 activations whose rows do not start on 16 bytes or that are sorted by group, and of bf16 ones whose shape TMA
+// cannot address.  64 x 64 tiles, 4 x 4 per thread.
 // With row counts: rows sorted by group, blockIdx.z = group, W = the groups' matrices one after another.
 #include "moe.cuh"
 #include "stack_common.cuh"
@@ -61,6 +62,10 @@ int gemm_any(const void* X, int x_dtype, const void* W, float* out, int M, int N
   if (!X || !W || !out || M <= 0 || N <= 0 || K <= 0 || (M + kSgT - 1) / kSgT > 65535) {
     set_last_error("bcg_gemm_any", "null pointer, non-positive dimension or M too large");
     return BCG_ERR_ARG;
+  }
+  if (x_dtype == BCG_DT_F32) {
+    const int rc = gemm_f32(static_cast<const float*>(X), W, out, M, N, K, ldx, ldw, ldo, st);
+    if (rc != BCG_ERR_UNSUPPORTED) return rc;
   }
   const dim3 grid((N + kSgT - 1) / kSgT, (M + kSgT - 1) / kSgT);
   const auto* w = static_cast<const __nv_bfloat16*>(W);

@@ -601,7 +601,7 @@ int grouped_in(const bcg_stack* m, const bcg_layer* l, const bcg_stack_ws* ws, c
 }
 
 // ------------------------------------------------------------------------------------------- plain
-constexpr int kGpThreads = 128, kGpKeys = 256;
+constexpr int kGpThreads = 512, kGpKeys = 256, kGpWarps = kGpThreads / 32, kGpAhead = 4;
 
 struct GroupedAttn {
   const void *q, *k_cache, *v_cache;
@@ -625,14 +625,23 @@ struct GroupedAttn {
   }
 };
 
+// Groups of threads that share the values' columns
+__host__ __device__ __forceinline__ int plain_groups(int dim, int vdim) {
+  const int n = vdim >= kGpThreads ? 1 : kGpThreads / ((vdim + 31) / 32 * 32);
+  return dim + n * vdim + kGpKeys > 16384 ? 1 : n;      // 64 KB of shared memory
+}
+
+// Keys' rows are looked up once per chunk, a warp has kGpAhead keys' reads in flight, and the values' columns are read by as many
+// groups of threads as the CTA has, a part of the keys each.  Single tokens at 410 keys, 16 heads: 80 -> 30 us.
 template <typename T>
 __global__ void __launch_bounds__(kGpThreads)
 grouped_plain_kernel(const GroupedAttn a) {
   extern __shared__ float sm[];
-  __shared__ float red[kGpThreads / 32];
+  __shared__ float red[kGpWarps];
+  __shared__ long long key_row[kGpKeys];
   float* qs = sm;             // [dim]
-  float* oc = qs + a.dim;     // [vdim]
-  float* p = oc + a.vdim;     // [kGpKeys]
+  float* p = qs + a.dim;      // [kGpKeys]
+  float* oc = p + kGpKeys;    // [groups][vdim]
   pdl_launch_dependents();
   pdl_wait();
   const long long t = a.rows ? a.rows[blockIdx.x] : blockIdx.x;
@@ -642,8 +651,10 @@ grouped_plain_kernel(const GroupedAttn a) {
   const int* bt = a.block_table + static_cast<long long>(a.row_seq ? a.row_seq[t] : t) * a.max_blocks;
   const T* qh = static_cast<const T*>(a.q) + (t * a.heads + h) * a.q_ld;
   const float slope = a.slopes ? a.slopes[h] : 0.f;
+  const int groups = plain_groups(a.dim, a.vdim), width = groups > 1 ? kGpThreads / groups : kGpThreads;
+  const int group = threadIdx.x / width, column = threadIdx.x % width;
   for (int i = threadIdx.x; i < a.dim; i += kGpThreads) qs[i] = to_f32<T>(qh[i]);
-  for (int i = threadIdx.x; i < a.vdim; i += kGpThreads) oc[i] = 0.f;
+  for (int i = threadIdx.x; i < groups * a.vdim; i += kGpThreads) oc[i] = 0.f;
   float m = -INFINITY, l = 0.f;
   const int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
   // tokens lo .. pos, then the pooled blocks that are seen
@@ -654,19 +665,30 @@ grouped_plain_kernel(const GroupedAttn a) {
   for (int j0 = 0; j0 < n_all; j0 += kGpKeys) {
     const int n = min(kGpKeys, n_all - j0);
     __syncthreads();
+    for (int j = threadIdx.x; j < n; j += kGpThreads) key_row[j] = row_of(j0 + j);
+    __syncthreads();
     float mx = -INFINITY;
-    for (int j = warp; j < n; j += kGpThreads / 32) {
-      const T* k = static_cast<const T*>(a.k_cache) + row_of(j0 + j) * a.q_ld;
-      float s = 0.f;
-      for (int i = lane; i < a.dim; i += 32) s = fmaf(qs[i], to_f32<T>(k[i]), s);
-      s = warp_sum(s) * a.scale - slope * static_cast<float>(pos - lo - (j0 + j));
-      if (lane == 0) p[j] = s;
-      mx = fmaxf(mx, s);
+    for (int j = warp * kGpAhead; j < n; j += kGpWarps * kGpAhead) {
+      const T* k[kGpAhead];
+      float s[kGpAhead] = {};
+#pragma unroll
+      for (int u = 0; u < kGpAhead; ++u) k[u] = static_cast<const T*>(a.k_cache) + key_row[min(j + u, n - 1)] * a.q_ld;
+#pragma unroll 4
+      for (int i = lane; i < a.dim; i += 32)
+#pragma unroll
+        for (int u = 0; u < kGpAhead; ++u) s[u] = fmaf(qs[i], to_f32<T>(k[u][i]), s[u]);
+#pragma unroll
+      for (int u = 0; u < kGpAhead; ++u) {
+        if (j + u >= n) break;
+        const float x = warp_sum(s[u]) * a.scale - slope * static_cast<float>(pos - lo - (j0 + j + u));
+        if (lane == 0) p[j + u] = x;
+        mx = fmaxf(mx, x);
+      }
     }
     if (lane == 0) red[warp] = mx;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kGpThreads / 32; ++i) mx = fmaxf(mx, red[i]);
+    for (int i = 0; i < kGpWarps; ++i) mx = fmaxf(mx, red[i]);
     const float m_new = fmaxf(m, mx);
     const float corr = expf(m - m_new);
     float sum = 0.f;
@@ -681,25 +703,166 @@ grouped_plain_kernel(const GroupedAttn a) {
     __syncthreads();
     sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < kGpThreads / 32; ++i) sum += red[i];
+    for (int i = 0; i < kGpWarps; ++i) sum += red[i];
     l = l * corr + sum;
     m = m_new;
-    for (int r = threadIdx.x; r < a.vdim; r += kGpThreads) {
-      float acc = oc[r] * corr;
-      for (int j = 0; j < n; ++j)
-        acc = fmaf(p[j], to_f32<T>(static_cast<const T*>(a.v_cache)[row_of(j0 + j) * a.v_ld + r]), acc);
-      oc[r] = acc;
-    }
+    if (group < groups)
+      for (int r = column; r < a.vdim; r += width) {
+        float acc = oc[group * a.vdim + r] * corr;
+#pragma unroll 8
+        for (int j = group; j < n; j += groups)
+          acc = fmaf(p[j], to_f32<T>(static_cast<const T*>(a.v_cache)[key_row[j] * a.v_ld + r]), acc);
+        oc[group * a.vdim + r] = acc;
+      }
   }
   __syncthreads();
   const float inv = (a.gates ? a.gates[t * a.heads + h] : 1.0f) / l;
   T* dst = static_cast<T*>(a.out) + t * a.out_ld + static_cast<long long>(h) * a.vdim;
+  auto total = [&](int r) {
+    float s = 0.f;
+    for (int i = 0; i < groups; ++i) s += oc[i * a.vdim + r];
+    return s * inv;
+  };
   for (int r = threadIdx.x * 2; r < a.vdim; r += kGpThreads * 2) {
-    float u = oc[r] * inv, v = r + 1 < a.vdim ? oc[r + 1] * inv : 0.f;
+    float u = total(r), v = r + 1 < a.vdim ? total(r + 1) : 0.f;
     a.turn_back(pos, r, u, v);
     dst[r] = from_f32<T>(u);
     if (r + 1 < a.vdim) dst[r + 1] = from_f32<T>(v);
   }
+}
+
+// ------------------------------------------------------------------------------------------- fp32, many tokens
+// A CTA has one head of 32 tokens that follow one another in the batch, a warp four of them, and 64 keys and values at a time in
+// shared memory.  A key that a lane reads serves four queries, and so does a value: one CTA per token (grouped_plain) read every
+// key from L2 again for each.  Tokens of several sequences in a CTA take their turns.  16 heads of 2 x 410 tokens: 1740 -> 115 us.
+constexpr int kGtThreads = 256, kGtQueries = 32, kGtKeys = 64, kGtDim = 128, kGtPitch = kGtDim + 4;
+constexpr int kGtSmem = (kGtQueries * kGtDim + kGtKeys * kGtPitch + kGtKeys * kGtDim + kGtQueries * kGtKeys) * 4;
+
+__global__ void __launch_bounds__(kGtThreads)
+grouped_tile_kernel(const GroupedAttn a, int n_tokens) {
+  extern __shared__ __align__(16) float sm[];
+  float* qs = sm;                               // [32][128]
+  float* ks = qs + kGtQueries * kGtDim;         // [64][132]: eight lanes' float4 fall on eight places
+  float* vs = ks + kGtKeys * kGtPitch;          // [64][128]
+  float* ps = vs + kGtKeys * kGtDim;            // [32][64]
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t0 = (gridDim.x - 1 - blockIdx.x) * kGtQueries, nq = min(kGtQueries, n_tokens - t0);     // the longest contexts first
+  const int h = blockIdx.y, g = h / (a.heads / a.kv_heads);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qw = warp * 4;
+  const float slope = a.slopes ? a.slopes[h] : 0.f;
+  const int d4 = a.dim / 4, v4 = a.vdim / 4;
+  for (int i = threadIdx.x; i < nq * d4; i += kGtThreads) {
+    const int r = i / d4, c = i % d4;
+    *reinterpret_cast<float4*>(qs + r * kGtDim + c * 4) =
+        *reinterpret_cast<const float4*>(static_cast<const float*>(a.q) + (static_cast<long long>(t0 + r) * a.heads + h) * a.q_ld + c * 4);
+  }
+  int pos[4];
+  float m[4], l[4];
+  float4 o[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    pos[u] = a.positions[t0 + min(qw + u, nq - 1)];
+    m[u] = -INFINITY;
+    l[u] = 0.f;
+    o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int s0 = 0; s0 < nq;) {      // tokens s0 .. s1 - 1 belong to one sequence
+    const int seq = a.row_seq[t0 + s0];
+    int s1 = s0 + 1, first = a.positions[t0 + s0], last = first;
+    for (; s1 < nq && a.row_seq[t0 + s1] == seq; ++s1) {
+      const int x = a.positions[t0 + s1];
+      first = min(first, x);
+      last = max(last, x);
+    }
+    const int* bt = a.block_table + static_cast<long long>(seq) * a.max_blocks;
+    const bool mine = qw < s1 && qw + 4 > s0;
+    for (int j0 = a.window > 0 ? max(0, first - a.window + 1) : 0; j0 <= last; j0 += kGtKeys) {
+      const int n = min(kGtKeys, last + 1 - j0);
+      __syncthreads();
+      for (int j = warp; j < kGtKeys; j += kGtThreads / 32) {
+        // rows behind the last key repeat it: they are masked below
+        const long long row = page_row(bt, 0, j0 + min(j, n - 1), a.kv_heads, g, a.page_size);
+        if (lane < d4)
+          *reinterpret_cast<float4*>(ks + j * kGtPitch + lane * 4) =
+              *reinterpret_cast<const float4*>(static_cast<const float*>(a.k_cache) + row * a.q_ld + lane * 4);
+        if (lane < v4)
+          *reinterpret_cast<float4*>(vs + j * kGtDim + lane * 4) =
+              *reinterpret_cast<const float4*>(static_cast<const float*>(a.v_cache) + row * a.v_ld + lane * 4);
+      }
+      __syncthreads();
+      if (!mine) continue;
+      float4 s[4][2];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u][0] = s[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < d4; ++i) {
+        const float4 k0 = *reinterpret_cast<const float4*>(ks + lane * kGtPitch + i * 4);
+        const float4 k1 = *reinterpret_cast<const float4*>(ks + (lane + 32) * kGtPitch + i * 4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 q = *reinterpret_cast<const float4*>(qs + (qw + u) * kGtDim + i * 4);
+          s[u][0].x = fmaf(q.x, k0.x, s[u][0].x); s[u][0].y = fmaf(q.y, k0.y, s[u][0].y);
+          s[u][0].z = fmaf(q.z, k0.z, s[u][0].z); s[u][0].w = fmaf(q.w, k0.w, s[u][0].w);
+          s[u][1].x = fmaf(q.x, k1.x, s[u][1].x); s[u][1].y = fmaf(q.y, k1.y, s[u][1].y);
+          s[u][1].z = fmaf(q.z, k1.z, s[u][1].z); s[u][1].w = fmaf(q.w, k1.w, s[u][1].w);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float x[2], top = -INFINITY;
+        bool seen[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int away = pos[u] - (j0 + lane + 32 * e);
+          seen[e] = qw + u >= s0 && qw + u < s1 && away >= 0 && (a.window <= 0 || away < a.window);
+          x[e] = ((s[u][e].x + s[u][e].y) + (s[u][e].z + s[u][e].w)) * a.scale - slope * static_cast<float>(away);
+          if (seen[e]) top = fmaxf(top, x[e]);
+        }
+        const float m_new = fmaxf(m[u], warp_max(top));
+        const float corr = m_new == m[u] ? 1.f : expf(m[u] - m_new);
+        float sum = 0.f;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float y = seen[e] ? expf(x[e] - m_new) : 0.f;
+          ps[(qw + u) * kGtKeys + lane + 32 * e] = y;
+          sum += y;
+        }
+        l[u] = l[u] * corr + warp_sum(sum);
+        m[u] = m_new;
+        o[u].x *= corr; o[u].y *= corr; o[u].z *= corr; o[u].w *= corr;
+      }
+      __syncwarp();
+      if (lane < v4) {
+#pragma unroll 4
+        for (int j = 0; j < kGtKeys; j += 4) {
+          float4 p[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) p[u] = *reinterpret_cast<const float4*>(ps + (qw + u) * kGtKeys + j);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float4 v = *reinterpret_cast<const float4*>(vs + (j + e) * kGtDim + lane * 4);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float y = e == 0 ? p[u].x : e == 1 ? p[u].y : e == 2 ? p[u].z : p[u].w;
+              o[u].x = fmaf(y, v.x, o[u].x); o[u].y = fmaf(y, v.y, o[u].y);
+              o[u].z = fmaf(y, v.z, o[u].z); o[u].w = fmaf(y, v.w, o[u].w);
+            }
+          }
+        }
+      }
+      __syncwarp();
+    }
+    s0 = s1;
+  }
+  if (lane >= v4) return;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (qw + u < nq) {
+      const long long t = t0 + qw + u;
+      const float inv = (a.gates ? a.gates[t * a.heads + h] : 1.0f) / l[u];
+      *reinterpret_cast<float4*>(static_cast<float*>(a.out) + t * a.out_ld + static_cast<long long>(h) * a.vdim + lane * 4) =
+          make_float4(o[u].x * inv, o[u].y * inv, o[u].z * inv, o[u].w * inv);
+    }
 }
 
 static GroupedAttn attn_args(const bcg_stack* m, const bcg_layer* l, const bcg_stack_ws* ws, const bcg_step_batch* b,
@@ -735,7 +898,16 @@ static GroupedAttn attn_args(const bcg_stack* m, const bcg_layer* l, const bcg_s
 static int grouped_plain(const bcg_stack* m, const bcg_layer* l, const bcg_stack_ws* ws, const bcg_step_batch* b,
                          const int* rows, int n, cudaStream_t st) {
   const GroupedAttn a = attn_args(m, l, ws, b, rows);
-  const int sm = (l->dim + l->vdim + kGpKeys) * 4;
+  // Prompts' tokens share keys; among tokens that each have a sequence of their own there is nothing to share.
+  if (m->act_dtype == BCG_DT_F32 && !rows && b->row_seq && n >= 2 * b->n_seqs && l->pool == 0 && !a.v_cos_sin && l->dim % 4 == 0 &&
+      l->vdim % 4 == 0 && l->dim <= kGtDim && l->vdim <= kGtDim && l->q_ld % 4 == 0 && l->v_ld % 4 == 0 && l->mix_ld % 4 == 0 &&
+      ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache) |
+        reinterpret_cast<uintptr_t>(a.out)) & 15) == 0) {
+    BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_tile_kernel), kGtSmem));
+    BCG_CUDA_CHECK(launch_k(grouped_tile_kernel, dim3((n + kGtQueries - 1) / kGtQueries, l->heads), dim3(kGtThreads), kGtSmem, st, a, n));
+    return BCG_OK;
+  }
+  const int sm = (l->dim + plain_groups(l->dim, l->vdim) * l->vdim + kGpKeys) * 4;
   const dim3 grid(n, l->heads);
   if (m->act_dtype == BCG_DT_F32) {
     BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_plain_kernel<float>), 64 * 1024));

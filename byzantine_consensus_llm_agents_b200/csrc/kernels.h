@@ -114,6 +114,9 @@ int sandwich_norm(float* residual, const float* delta, int n_partials, long long
                   const NormExtra& extra, cudaStream_t stream);
 int poly_norm(const float* z, int n_partials, long long partial_stride, const float* coef, void* out, int act_dtype,
               int T, int ff, float eps, cudaStream_t stream);
+// fp32 activations on tensor cores, or a few rows of them; BCG_ERR_UNSUPPORTED: rows do not start on 16 bytes
+int gemm_f32(const float* X, const void* W, float* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
+             cudaStream_t st);
 int gemm_any(const void* X, int x_dtype, const void* W, float* out, int M, int N, int K, long long ldx,
              long long ldw, long long ldo, cudaStream_t stream);
 int latent_qkv(const bcg_layer* l, const float* proj, int n_partials, long long pstride, const int* positions,

@@ -146,6 +146,15 @@ def test_grouped_attention_fp32(size, window):
     _check(a, _seqs(a, ((300, 20), (40, 40), (9, 1)), window), 3e-6)
 
 
+@pytest.mark.parametrize("size", ["small", "usual", "max"])
+@pytest.mark.parametrize("window", [0, 1, 33, 65])
+def test_grouped_attention_fp32_tiles(size, window):
+    """Thirty-two tokens of one or several sequences per CTA, 64 keys at a time: ends of both inside and between sequences.  A row is a
+    softmax average, so its error is a few units of fp32 times the scores' size, as with one token per CTA."""
+    a = Attention(size, window, "float32")
+    _check(a, _seqs(a, ((130, 33), (65, 64), (64, 1), (40, 3), (31, 31)), window), 3e-6)
+
+
 @pytest.mark.parametrize("context", [1, 15, 16, 17, 333, 2000])
 @pytest.mark.parametrize("window", [0, 700])
 def test_single_tokens_at_many_cluster_sizes(context, window):

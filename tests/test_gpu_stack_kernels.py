@@ -318,3 +318,34 @@ def test_sink_takes_its_share(size):
     keep = a.sink
     a.sink = torch.full_like(keep, -1e4)
     assert ((torch.stack([a.oracle(*x) for x in meta]) - out.double()).norm() / out.double().norm()) > 1.0
+
+
+# Rows that start on 16 bytes: streamed rows up to four, then tensor-core tiles of 128 and of 32 columns, remainders in each direction.
+# An output is a sum of K products in fp32: K + 1 roundings of at most the sum of the products' sizes bound it, sqrt(K) of them are expected.
+@pytest.mark.parametrize("M,N,K", [(1, 9, 8), (2, 70, 1032), (3, 8, 2056), (4, 129, 64), (5, 33, 72), (127, 31, 200), (128, 2048, 136),
+                                   (129, 130, 64), (300, 2500, 192), (260, 12320, 64)])
+def test_gemm_any_aligned_rows(M, N, K):
+    g = gen(M + N + K)
+    x, w = torch.randn(M, K, generator=g) * torch.exp2(torch.randint(-20, 20, (M, K), generator=g).float()), torch.randn(N, K, generator=g).bfloat16()
+    for ldo in (N + 3, (N + 3) // 4 * 4):
+        out = torch.full((M, ldo), 7.0, device="cuda")
+        X, W = dev(x), dev(w)
+        L.check(L.load().bcg_gemm_any(X.data_ptr(), L.DT_F32, W.data_ptr(), out.data_ptr(), M, N, K, K, K, ldo, L.stream_ptr()))
+        got, xd, wd = out[:, :N].double().cpu(), x.double(), w.double()
+        assert ((got - xd @ wd.T).abs() <= 4 * K ** 0.5 * 2 ** -24 * (xd.abs() @ wd.abs().T)).all()
+        assert (out[:, N:] == 7.0).all()
+
+
+def test_gemm_any_keeps_infinities_and_nans():
+    g = gen(0)
+    x, w = torch.randn(40, 512, generator=g), torch.randn(64, 512, generator=g).bfloat16()
+    x[3, 5], x[7, 9], x[8, 1], x[9, 2] = float("inf"), float("nan"), 3.0e38, 1e-41
+    w[:, 1] = 0.5
+    for rows in (slice(0, 40), slice(6, 10)):
+        X, W = dev(x[rows]), dev(w)
+        out = torch.zeros(len(X), 64, device="cuda")
+        L.check(L.load().bcg_gemm_any(X.data_ptr(), L.DT_F32, W.data_ptr(), out.data_ptr(), len(X), 64, 512, 512, 512, 64, L.stream_ptr()))
+        want = (x[rows].double() @ w.double().T).float()
+        assert torch.equal(out.isnan().cpu(), want.isnan()) and torch.equal(out.isinf().cpu(), want.isinf())
+        ok = want.isfinite()
+        torch.testing.assert_close(out.cpu()[ok], want[ok], rtol=1e-5, atol=1e-4)
