@@ -249,6 +249,7 @@ delta_token_kernel(const DeltaArgs a, T* __restrict__ out) {
   const int cta = CL > 1 ? static_cast<int>(blockIdx.x) : 0;
   const int h = blockIdx.y, t = blockIdx.z;
   pdl_launch_dependents();
+  row_sum_begin(sh);
   // Positions, slots and the state were written by earlier steps, which are complete before any kernel of
   // this step starts (a step's first launch follows the sampler's bookkeeping kernel or a copy, neither of
   // which lets its successor start early), so the state is on its way while the projections are finished.
@@ -260,6 +261,7 @@ delta_token_kernel(const DeltaArgs a, T* __restrict__ out) {
   if (idle || fresh) S.zero();
   else S.load(st, D, rg, col);
   pdl_wait();
+  row_sum_ready<CL>();
   if (idle) return;                                     // the same for the whole cluster
   {   // raw projections: a thread's elements and up to four slabs of each in flight together
     constexpr int kE = (6 * DP + kTokThreads - 1) / kTokThreads;
@@ -333,14 +335,14 @@ delta_token_kernel(const DeltaArgs a, T* __restrict__ out) {
       so[lcol + c] = o[c];
       if (col + c < D) ss[0] += o[c] * o[c];
     }
-  row_sum<kTokThreads, CL, 1>(sh, ss, 0);               // also orders `so`
+  __syncthreads();                                      // `so`
+  row_sum<kTokThreads, CL, 1>(sh, ss, 0);
   const float inv = rsqrtf(ss[0] / static_cast<float>(D) + a.eps);
   for (int i = threadIdx.x; i < kCols; i += kTokThreads) {
     const int ch = cta * kCols + i;
     if (ch < D)
       out[static_cast<long long>(t) * HD + h * D + ch] = from_f32<T>(so[i] * inv * a.out_norm[h * D + ch] * op[5 * DP + ch]);
   }
-  row_sum_exit<CL>();
 }
 
 template <typename T, int DP, int CPT>

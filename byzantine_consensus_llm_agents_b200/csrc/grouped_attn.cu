@@ -144,7 +144,9 @@ grouped_norm_in_kernel(const GroupedIn a) {
   float* stage = reinterpret_cast<float*>(stage_raw);
   __shared__ RowSum<kInThreads, CL, 2> sh;
   pdl_launch_dependents();
+  row_sum_begin(sh);
   pdl_wait();
+  row_sum_ready<CL>();
   const int cta = CL > 1 ? static_cast<int>(blockIdx.x) : 0;
   const InToken tok(a, CL > 1 ? blockIdx.y : blockIdx.x);
   const float* row = a.proj + tok.t * a.ld;
@@ -176,7 +178,6 @@ grouped_norm_in_kernel(const GroupedIn a) {
     }
     store_columns<T, V>(a, tok, c, x);
   }
-  row_sum_exit<CL>();
 }
 
 template <typename T, int V>

@@ -103,53 +103,78 @@ __device__ __forceinline__ Vec<V> slab_sum_vec(const float* p, int n, long long 
 
 // Sum of N values over the THREADS x CL threads that share a row (CL CTAs of one cluster); fixed order, so a
 // row's result does not depend on its neighbours.  `slot` must be a fresh 0, 1, ... per call in a kernel.
-// Before a kernel with CL > 1 ends, every thread must pass row_sum_exit<CL>().
+//
+// In a cluster every warp sends its sums to every CTA, whose threads wait for the bytes on a barrier of their own: one way
+// through distributed shared memory.  (A barrier of the cluster and eight remote reads behind it took two and the CTA's own barrier.)
+// row_sum_begin comes first, all threads then pass row_sum_ready in front of the first sum (the peers' barriers exist), and only
+// the first `warps` warps of each CTA take part in sums.  Who takes part in the last sum of a kernel may leave behind it: all that
+// is sent to a CTA has arrived when its threads go on.
 template <int THREADS, int CL, int N>
 struct RowSum {
-  float warp[N][THREADS / 32];
-  float cta[2][N];
+  static constexpr int kWarps = THREADS / 32;
+  float warp[CL > 1 ? 2 : 1][N][CL * kWarps];
+  uint64_t bar[2];
 };
 template <int THREADS, int CL, int N>
-__device__ __forceinline__ void row_sum(RowSum<THREADS, CL, N>& sh, float (&v)[N], int slot) {
+__device__ __forceinline__ void row_sum_begin(RowSum<THREADS, CL, N>& sh, int warps = THREADS / 32) {
+  if constexpr (CL > 1) {
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&sh.bar[i], 1);
+        mbar_arrive_expect_tx(&sh.bar[i], static_cast<uint32_t>(CL * warps * N * 4));
+      }
+      fence_barrier_init();
+    }
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  }
+}
+template <int CL>
+__device__ __forceinline__ void row_sum_ready() {
+  if constexpr (CL > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+template <int THREADS, int CL, int N>
+__device__ __forceinline__ void row_sum(RowSum<THREADS, CL, N>& sh, float (&v)[N], int slot, int warps = THREADS / 32) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    v[k] = warp_sum(v[k]);
-    if (lane == 0) sh.warp[k][warp] = v[k];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    float t = 0.f;
-#pragma unroll
-    for (int i = 0; i < THREADS / 32; ++i) t += sh.warp[k][i];
-    v[k] = t;
-  }
+  for (int k = 0; k < N; ++k) v[k] = warp_sum(v[k]);
   if constexpr (CL > 1) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    if (threadIdx.x < N) {
-      float mine = v[0];
+    uint32_t rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    if (lane < CL) {
 #pragma unroll
-      for (int k = 1; k < N; ++k)
-        if (static_cast<int>(threadIdx.x) == k) mine = v[k];
-      sh.cta[slot & 1][threadIdx.x] = mine;
+      for (int k = 0; k < N; ++k)
+        asm volatile(
+            "{\n"
+            ".reg .b32 dst, bar;\n"
+            "mapa.shared::cluster.u32 dst, %0, %2;\n"
+            "mapa.shared::cluster.u32 bar, %1, %2;\n"
+            "st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [dst], %3, [bar];\n"
+            "}\n" ::"r"(smem_u32(&sh.warp[slot & 1][k][rank * warps + warp])),
+            "r"(smem_u32(&sh.bar[slot & 1])), "r"(lane), "r"(__float_as_uint(v[k]))
+            : "memory");
     }
-    cluster.sync();
+    mbar_wait(&sh.bar[slot & 1], 0);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      float t = 0.f;
+      for (int i = lane; i < CL * warps; i += 32) t += sh.warp[slot & 1][k][i];
+      v[k] = warp_sum(t);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (lane == 0) sh.warp[0][k][warp] = v[k];
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       float t = 0.f;
 #pragma unroll
-      for (int i = 0; i < CL; ++i) t += *cluster.map_shared_rank(&sh.cta[slot & 1][k], i);
+      for (int i = 0; i < THREADS / 32; ++i) t += sh.warp[0][k][i];
       v[k] = t;
     }
-  } else {
     __syncthreads();
   }
-}
-template <int CL>
-__device__ __forceinline__ void row_sum_exit() {
-  if constexpr (CL > 1) cooperative_groups::this_cluster().sync();
 }
 
 template <typename... KArgs, typename... Args>

@@ -78,6 +78,20 @@ def test_poly_norm(dtype, T, ff, parts):
         close(out, R.poly_norm(z.double().sum(0), coef, 1e-5), tol)
 
 
+# Rows over clusters: one, two and four threads per vector, the widest row of each, slabs fewer and more than threads, and the
+# next width, which the general kernel takes.
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("T,d,parts", [(6, 1024, 1), (4, 2052, 14), (128, 2048, 3), (3, 4096, 9), (2, 8192, 16), (1, 8196, 2)])
+def test_sandwich_norm_of_few_rows(dtype, T, d, parts):
+    test_sandwich_norm(dtype, T, d, parts)
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("T,ff,parts", [(2, 1024, 1), (128, 7424, 5), (3, 8192, 16), (2, 8196, 2), (1, 16384, 3), (1, 16388, 2)])
+def test_poly_norm_of_few_rows(dtype, T, ff, parts):
+    test_poly_norm(dtype, T, ff, parts)
+
+
 # ------------------------------------------------------------------------------------------ delta rule
 class Delta:
     """One delta-rule layer's operands for ragged sequences, and the oracle's answer."""
