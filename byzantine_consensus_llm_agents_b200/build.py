@@ -22,6 +22,7 @@ LIB_TIMELINE = OUT / "libbcg_b200_tl.so"
 
 SOURCES = [
     "capi.cu",
+    "block_hash.cu",
     "gemm_tcgen05.cu",
     "gemm2sm_tcgen05.cu",
     "norm_rope.cu",

@@ -216,6 +216,8 @@ int bcg_stack_head(const bcg_stack* m, const bcg_stack_ws* ws, const int* rows, 
   return stack_head(m, ws, rows, n, row0, flags, S(stream));
 }
 
+int bcg_block_hashes(const int* tokens, int n_blocks, int block, unsigned char* out) { return block_hashes(tokens, n_blocks, block, out); }
+
 int bcg_gemm_any(const void* X, int x_dtype, const void* W, float* out, int M, int N, int K, long long ldx,
                  long long ldw, long long ldo, void* stream) {
   return gemm_any(X, x_dtype, W, out, M, N, K, ldx, ldw, ldo, S(stream));

@@ -114,6 +114,8 @@ int sandwich_norm(float* residual, const float* delta, int n_partials, long long
                   const NormExtra& extra, cudaStream_t stream);
 int poly_norm(const float* z, int n_partials, long long partial_stride, const float* coef, void* out, int act_dtype,
               int T, int ff, float eps, cudaStream_t stream);
+// block_hash.cu
+int block_hashes(const int* tokens, int n_blocks, int block, unsigned char* out);
 // fp32 activations on tensor cores, or a few rows of them; BCG_ERR_UNSUPPORTED: rows do not start on 16 bytes
 int gemm_f32(const float* X, const void* W, float* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
              cudaStream_t st);

@@ -94,6 +94,28 @@ class PagePool:
     def chain(prev: bytes, block: Sequence[int]) -> bytes:
         return hashlib.blake2b(prev + struct.pack(f"<{len(block)}i", *block), digest_size=16).digest()
 
+    @staticmethod
+    def chains(ids: Sequence[int]) -> Sequence[bytes]:
+        """chain() over all full blocks of a prompt, in one native call."""
+        n = len(ids) // PAGE
+        if not n:
+            return ()
+        out = C.create_string_buffer(16 * n)
+        L.check(L.load().bcg_block_hashes(struct.pack(f"<{n * PAGE}i", *ids[:n * PAGE]), n, PAGE, out), "bcg_block_hashes")
+        return struct.unpack("16s" * n, out.raw)
+
+    def acquire_prefix(self, hashes: Sequence[bytes]) -> List[int]:
+        """The pages of the longest cached run of these blocks, each held once more."""
+        cached, ref, pages = self.cached, self.ref, []
+        for h in hashes:
+            p = cached.get(h)
+            if p is None:
+                break
+            cached.move_to_end(h)
+            ref[p] = ref.get(p, 0) + 1
+            pages.append(p)
+        return pages
+
     def lookup(self, h: bytes) -> Optional[int]:
         p = self.cached.get(h)
         if p is not None:
@@ -391,22 +413,11 @@ class Engine:
         # ---- page layout + prefix-cache lookup
         try:
             for ids, q in zip(ids_list, reqs):
-                n_full = len(ids) // PAGE
-                hs, h = [], b"\0" * 16
-                for j in range(n_full):
-                    h = PagePool.chain(h, ids[j * PAGE:(j + 1) * PAGE])
-                    hs.append(h)
-                pages, hit = [], 0
+                hs, pages = (), []
                 if self.enable_prefix_cache:
-                    for j in range(n_full):
-                        if (j + 1) * PAGE >= len(ids):
-                            break  # always compute at least the last prompt token
-                        p = self.pool.lookup(hs[j])
-                        if p is None:
-                            break
-                        self.pool.acquire(p)
-                        pages.append(p)
-                        hit += 1
+                    hs = PagePool.chains(ids)
+                    pages = self.pool.acquire_prefix(hs[:(len(ids) - 1) // PAGE])   # always compute at least the last prompt token
+                hit = len(pages)
                 total_pages = (len(ids) + q.max_tokens + PAGE - 1) // PAGE
                 while len(pages) < total_pages:
                     pages.append(self.pool.alloc())

@@ -182,6 +182,7 @@ _SIGS = {
                                    C.c_int, C.c_int, C.c_int, vp]),
     "bcg_stack_step": (C.c_int, [C.POINTER(Stack), C.POINTER(StackWs), C.POINTER(StepBatch), vp]),
     "bcg_stack_head": (C.c_int, [C.POINTER(Stack), C.POINTER(StackWs), vp, C.c_int, C.c_int, C.c_int, vp]),
+    "bcg_block_hashes": (C.c_int, [C.c_char_p, C.c_int, C.c_int, C.c_char_p]),
     "bcg_gemm_any": (C.c_int, [vp, C.c_int, vp, vp, C.c_int, C.c_int, C.c_int, C.c_longlong, C.c_longlong,
                                C.c_longlong, vp]),
     "bcg_sandwich_norm": (C.c_int, [vp, vp, C.c_int, C.c_longlong, vp, vp, vp, C.c_int, C.c_int, C.c_int, C.c_float,

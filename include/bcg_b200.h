@@ -572,7 +572,8 @@ int bcg_stack_head(const bcg_stack* m, const bcg_stack_ws* ws, const int* rows, 
 
 /* The mechanisms one by one (what bcg_stack_step launches; the reference has no counterpart).
  * `in` arguments with n_partials slabs are fp32 split-K outputs added in index order. */
-/* out fp32 [M, ldo] = X [M, ldx] (act_dtype) * W bf16 [N, ldw]^T on CUDA cores, any shape. */
+/* out fp32 [M, ldo] = X [M, ldx] (act_dtype) * W bf16 [N, ldw]^T in fp32, any shape: on tensor cores where X is
+ * fp32 and rows start on 16 bytes, on CUDA cores elsewhere. */
 int bcg_gemm_any(const void* X, int x_dtype, const void* W, float* out, int M, int N, int K, long long ldx,
                  long long ldw, long long ldo, void* stream);
 /* No counterpart in the reference: residual += w_post ? rmsnorm(delta) * w_post : delta, then
@@ -652,6 +653,11 @@ int bcg_expert_in(const bcg_stack* m, const bcg_stack_ws* ws, int layer, int T, 
  * ws->proj just the input and forget gates: what bcg_stack_step does in launches of more than 128 tokens. */
 int bcg_matrix_memory(const bcg_stack* m, const bcg_stack_ws* ws, const bcg_step_batch* b, int layer, int n_partials,
                       long long partial_stride, long long ld, int mode, void* stream);
+
+/* Host work, no counterpart of its own in the reference (the nearest is vLLM's prefix cache): 16-byte hash of every full block of
+ * `block` tokens (1..28), each a BLAKE2b over the previous block's hash (zeros in front of the first) and the tokens.
+ * tokens [n_blocks * block] and out [n_blocks * 16] are host memory. */
+int bcg_block_hashes(const int* tokens, int n_blocks, int block, unsigned char* out);
 
 #ifdef __cplusplus
 }

@@ -123,6 +123,24 @@ def test_page_pool_prefix_cache_and_eviction():
     assert pool.lookup(h1) is None
 
 
+def test_block_hashes_equal_the_chain():
+    from byzantine_consensus_llm_agents_b200.engine import PAGE, PagePool
+    for n in (0, 1, PAGE - 1, PAGE, PAGE + 1, 5 * PAGE, 1000):
+        ids = np.random.default_rng(n).integers(-2 ** 31, 2 ** 31, n).tolist()
+        want, h = [], b"\0" * 16
+        for j in range(n // PAGE):
+            h = PagePool.chain(h, ids[j * PAGE:(j + 1) * PAGE])
+            want.append(h)
+        assert list(PagePool.chains(ids)) == want
+    pool = PagePool(4)
+    hs = PagePool.chains(list(range(3 * PAGE)))
+    pages = [pool.alloc() for _ in range(2)]
+    for p, h in zip(pages, hs):
+        pool.publish(p, h)
+    assert pool.acquire_prefix(hs) == pages and [pool.ref[p] for p in pages] == [2, 2]
+    assert pool.acquire_prefix(hs[1:]) == pages[1:] and pool.acquire_prefix(hs[2:]) == []
+
+
 def test_row_seed_matches_oracle_restatement():
     from byzantine_consensus_llm_agents_b200.engine import row_seed
     from oracle.engine import row_seed as oracle_seed
