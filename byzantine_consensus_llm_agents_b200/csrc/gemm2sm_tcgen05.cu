@@ -46,10 +46,11 @@ struct Gemm2Args {
   int M, N, K;
   int tiles_m, tiles_n;   // 256-row / 256-column tiles
   int k_blocks;
+  int splits;             // of K, BCG_EPI_F32 only: slab s of the output lies s * slab elements behind the first
   int group_m;
   int epi;
   void* out;
-  long long ld_out;
+  long long ld_out, slab;
   float glu_limit, glu_alpha;   // BCG_EPI_GLU
   int sector_stores;         // fp32 output rows are 32-byte aligned: whole sectors per store
   uint64_t hint_a, hint_b;   // L2 eviction priority of the activation / weight loads
@@ -163,9 +164,11 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 
   const int n_clusters = gridDim.x >> 1;
   const int cluster_id = blockIdx.x >> 1;
-  const int total = args.tiles_m * args.tiles_n;
+  const int total = args.tiles_m * args.tiles_n * args.splits;
   const int group_tiles = args.group_m * args.tiles_n;
-  auto decode_item = [&](int item, int& tm, int& tn) {
+  auto decode_item = [&](int item, int& tm, int& tn, int& split) {
+    split = item % args.splits;
+    item /= args.splits;
     const int g = item / group_tiles;
     const int r = item - g * group_tiles;
     const int m0 = g * args.group_m;
@@ -174,6 +177,8 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     tm = m0 + (r - tn * gm);
   };
 
+  auto first_block = [&](int split) { return static_cast<int>(static_cast<long long>(split) * args.k_blocks / args.splits); };
+
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
     if (elect_one()) {      // one elected thread per role: see gemm_tcgen05.cu
@@ -181,11 +186,12 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       int stage = 0;
       uint32_t phase = 0;
       for (int item = cluster_id; item < total; item += n_clusters) {
-        int tm, tn;
-        decode_item(item, tm, tn);
+        int tm, tn, split;
+        decode_item(item, tm, tn, split);
+        const int kb1 = first_block(split + 1);
         const int row_a = tm * 256 + static_cast<int>(rank) * k2BlockM;
         const int row_b = tn * k2BlockN + static_cast<int>(rank) * (k2BlockN / 2);
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
+        for (int kb = first_block(split); kb < kb1; ++kb) {
           uint8_t* sa = smem + stage * k2StageBytes;
           mbar_wait(&empty_bar[stage], phase ^ 1);
           if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * k2StageBytes);
@@ -210,16 +216,17 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         mbar_wait(&tmem_empty[acc], acc_phase ^ 1);
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * k2BlockN);
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
+        const int split = item % args.splits, kb0 = first_block(split), kb1 = first_block(split + 1);
+        for (int kb = kb0; kb < kb1; ++kb) {
           mbar_wait(&full_bar[stage], phase);
           tc_fence_after();
           const uint64_t da = desc0 + static_cast<uint64_t>(stage * (k2StageBytes >> 4));
           const uint64_t db = da + (k2ABytes >> 4);
 #pragma unroll
           for (int k = 0; k < k2BlockK / 16; ++k)
-            umma_bf16_2sm(tmem_d, da + 2 * k, db + 2 * k, k2Idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_bf16_2sm(tmem_d, da + 2 * k, db + 2 * k, k2Idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           umma_commit_2sm(&empty_bar[stage]);
-          if (kb == args.k_blocks - 1) umma_commit_2sm(&tmem_full[acc]);
+          if (kb == kb1 - 1) umma_commit_2sm(&tmem_full[acc]);
           if (++stage == k2Stages) {
             stage = 0;
             phase ^= 1;
@@ -239,8 +246,8 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const int M = args.M, N = args.N;
     const long long ld = args.ld_out;
     for (int item = cluster_id; item < total; item += n_clusters) {
-      int tm, tn;
-      decode_item(item, tm, tn);
+      int tm, tn, split;
+      decode_item(item, tm, tn, split);
       mbar_wait(&tmem_full[acc], acc_phase);
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * k2BlockN);
@@ -286,7 +293,7 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           tmem_ld_x16(taddr + c + 16, v1);
           tmem_ld_wait();
           if (args.epi == BCG_EPI_F32) {
-            float* o = reinterpret_cast<float*>(args.out);
+            float* o = reinterpret_cast<float*>(args.out) + split * args.slab;
             if (m < M && n0 + c < N) {
               float4* dst = reinterpret_cast<float4*>(o + m * ld + n0 + c);
               if (args.sector_stores) {
@@ -352,13 +359,48 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   if (warp == 1) tmem_dealloc_2sm(tmem_base, k2TmemCols);
 }
 
-// Returns BCG_ERR_UNSUPPORTED when the shape is not for this kernel (the caller then uses the
-// single-CTA kernel).
-int gemm2sm_bf16_tn(const void* X, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,
-                    long long ld_out, int epi, float glu_limit, float glu_alpha, cudaStream_t stream) {
-  // the last column tile may be partial (the epilogue stores 32 columns at a time), where that wastes little
+static int pairs_of_sms() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms / 2;
+}
+
+// the last column tile may be partial (the epilogue stores 32 columns at a time), where that wastes little
+static bool for_pairs(int M, int N) {
   const int idle = (N + k2BlockN - 1) / k2BlockN * k2BlockN - N;
-  if (M < 512 || (N % 32) != 0 || idle * 8ll > N) return BCG_ERR_UNSUPPORTED;
+  return M > 128 && N % 32 == 0 && idle * 8ll <= N;
+}
+
+// A launch of one round takes 11.5 us and 0.28 us per k-block (launch, first reads, last stores; few rows are bound by 60 bytes per
+// clock and SM out of L2).  256 x 4096 -> 4096 in 1 / 2 / 4 parts: 29.8 / 21.5 / 17.8 us, 12288 -> 4096: 65.7 / 40.0 / 31.4; with
+// 951 rows 31.5 / 31.5 / 37.7 and 74.4 / 76.3 / 78.4, so that they stay whole.
+//
+// How many parts of K the fp32 product of a long launch is best cut into, where the consumer adds slabs: tiles that leave pairs of
+// SMs idle in the last round cost more than the slabs do.  Clocks: 520 per k-block and round (measured over 12 k rows; the MMAs
+// take 512), slabs written and read at about 4 KB per clock.  At most `room` floats of output.
+int gemm_long_splits(int M, int N, int K, long long room) {
+  if (!for_pairs(M, N)) return 1;
+  const int tiles = (M + 255) / 256 * ((N + k2BlockN - 1) / k2BlockN), kb = (K + k2BlockK - 1) / k2BlockK, pairs = pairs_of_sms();
+  const double slab = static_cast<double>(M) * N * 8.0 / 4096.0;
+  int best = 1;
+  double least = 0.0;
+  for (int s = 1; s <= 8 && static_cast<long long>(s) * M * N <= room && (s == 1 || kb / s >= 8); ++s) {
+    const double cost = 520.0 * ((tiles * s + pairs - 1) / pairs) * ((kb + s - 1) / s) + slab * s;
+    if (s == 1 || cost < 0.95 * least) {
+      best = s;
+      least = cost;
+    }
+  }
+  return best;
+}
+
+// Returns BCG_ERR_UNSUPPORTED when the shape is not for this kernel (the caller then uses the
+// single-CTA kernel).  From 129 rows on: up to 511 the single-CTA kernel's 128 x 256 tiles ran before, which read 48 KB per
+// k-block and SM where a pair's CTA reads 32 KB for as much work.
+int gemm2sm_bf16_tn(const void* X, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,
+                    long long ld_out, int epi, int splits, float glu_limit, float glu_alpha, cudaStream_t stream) {
+  if (!for_pairs(M, N) || (splits > 1 && epi != BCG_EPI_F32)) return BCG_ERR_UNSUPPORTED;
   static const bool off = getenv("BCG_GEMM_2SM") && atoi(getenv("BCG_GEMM_2SM")) == 0;   // tuning knob
   if (off) return BCG_ERR_UNSUPPORTED;
   Gemm2Args a = {};
@@ -380,22 +422,21 @@ int gemm2sm_bf16_tn(const void* X, const void* W, void* out, int M, int N, int K
   const uint64_t hints[3] = {kEvictNormal, kEvictFirst, kEvictLast};
   a.hint_a = hints[ha < 0 || ha > 2 ? 2 : ha];
   a.hint_b = hints[hb < 0 || hb > 2 ? 0 : hb];
+  a.splits = splits < a.k_blocks ? splits : a.k_blocks;
   a.epi = epi;
   a.out = out;
   a.ld_out = ld_out;
+  a.slab = static_cast<long long>(M) * ld_out;
   a.glu_limit = glu_limit;
   a.glu_alpha = glu_alpha;
-  a.sector_stores = (reinterpret_cast<uintptr_t>(out) % 32 == 0 && ld_out % 8 == 0) ? 1 : 0;
+  a.sector_stores = (reinterpret_cast<uintptr_t>(out) % 32 == 0 && ld_out % 8 == 0) ? 1 : 0;     // slabs then are, too
   CUtensorMap tma, tmb;
   int rc;
   if ((rc = make_tmap_bf16_sw128(&tma, X, M, K, ldx, k2BlockM)) != BCG_OK) return rc;
   if ((rc = make_tmap_bf16_sw128(&tmb, W, N, K, ldw, k2BlockN / 2)) != BCG_OK) return rc;
 
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int clusters = sms / 2;
-  const int total = a.tiles_m * a.tiles_n;
+  int clusters = pairs_of_sms();
+  const int total = a.tiles_m * a.tiles_n * a.splits;
   if (clusters > total) clusters = total;
   if (stages != 6) {
     if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(gemm2sm_tcgen05_kernel<7>), smem_2sm(7)))) return rc;

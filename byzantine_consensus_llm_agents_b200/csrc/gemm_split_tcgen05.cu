@@ -225,8 +225,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const SplitArgs a)
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// Activations are read with plain loads, here and above: a kernel that starts before its predecessor ends finds what a still
-// earlier one left in the read-only cache of its SM (two heads' products behind one another read the first one's rows again).
+// Activations are read with plain loads, here and above: read-only ones may be moved in front of the wait for the predecessor, as
+// nothing in the kernel can change what they read (two heads' products behind one another got the first one's rows again).
 
 // A few rows: weights stream through registers, eight output columns per CTA, the inputs split over four warps.  Two rows of
 // 2048 -> 12288: 182 -> 22 us (64 x 64 tiles waited for every 16 inputs' reads), of 11264 -> 2048: 771 -> 20 us.

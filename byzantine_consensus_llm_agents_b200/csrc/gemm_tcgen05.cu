@@ -714,9 +714,9 @@ static int gemm_dense(const void* X, const void* W, void* out, int M, int N, int
     set_last_error("bcg_gemm_bf16_tn", "ld_out must keep 16-byte row alignment");
     return BCG_ERR_ARG;
   }
-  if (!swap && splits == 1 && !(fu && (fu->scale_sumsq || fu->red_counters))) {
+  if (!swap && !(fu && (fu->scale_sumsq || fu->red_counters))) {
     // prefill-sized: 256x256 tiles on CTA pairs when the shape allows it
-    const int rc2 = gemm2sm_bf16_tn(X, W, out, M, N, K, ldx, ldw, ld_out, epi, glu_limit, glu_alpha, stream);
+    const int rc2 = gemm2sm_bf16_tn(X, W, out, M, N, K, ldx, ldw, ld_out, epi, splits, glu_limit, glu_alpha, stream);
     if (rc2 != BCG_ERR_UNSUPPORTED) return rc2;
   }
   GemmArgs a = {};

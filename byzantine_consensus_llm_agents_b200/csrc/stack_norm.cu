@@ -92,7 +92,12 @@ sandwich_norm_kernel(float* __restrict__ residual, const float* __restrict__ del
   for (int v = v0 + threadIdx.x * V; v < v1; v += kRowT * V) {
     Vec<V> y;
     if (delta) {
-      y = slab_sum_vec<V>(delta + t * d + v, n_partials, partial_stride);
+      if constexpr (CL > 1) {
+        y = slab_sum_vec<V>(delta + t * d + v, n_partials, partial_stride);
+      } else {      // a long launch's few slabs: other rows cover the reads, and slab_sum_vec's batch would mostly repeat the last
+        y = load_vec<V>(delta + t * d + v);
+        for (int s = 1; s < n_partials; ++s) y.add(load_vec<V>(delta + t * d + v + s * partial_stride));
+      }
     } else {
 #pragma unroll
       for (int k = 0; k < V; ++k) y.x[k] = 0.f;

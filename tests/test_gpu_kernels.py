@@ -702,3 +702,19 @@ def _check_prefill_attn(H, HKV, spec, q_scale):
         err = (got - ref).abs().max().item()
         assert err <= 3e-2, f"seq {b} err {err}"  # P rounded to bf16 before PV + bf16 output
         row += n
+
+
+# Long launches on pairs of SMs: the first row that they take, ends of tiles in each direction, K in parts of unequal length.  Slabs
+# are sums of bf16 products in fp32; together they are as close to 64 bits as the unsplit product.
+@pytest.mark.parametrize("M,N,K,splits", [(129, 256, 512, 1), (129, 256, 512, 3), (256, 288, 4096, 8), (257, 512, 1000, 2),
+                                          (511, 2048, 2048, 5), (700, 224, 136, 3), (1025, 1056, 640, 4)])
+def test_long_gemm_splits(M, N, K, splits):
+    g = torch.Generator().manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=g).bfloat16(), (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16()
+    out = torch.full((splits + 1, M, N), 7.0, device="cuda")
+    X, W = x.cuda(), w.cuda()
+    L.check(L.load().bcg_gemm_bf16_tn(X.data_ptr(), W.data_ptr(), out.data_ptr(), M, N, K, K, K, N, L.EPI_F32, splits, 0, L.stream_ptr()))
+    want = x.double() @ w.double().T
+    err = (out[:splits].double().sum(0).cpu() - want).abs().max().item()
+    assert err < 2e-5 * max(1.0, want.abs().max().item()), err      # K products of unit size, each sum rounded to 2^-24 of a few units
+    assert (out[splits] == 7.0).all()
