@@ -92,12 +92,7 @@ sandwich_norm_kernel(float* __restrict__ residual, const float* __restrict__ del
   for (int v = v0 + threadIdx.x * V; v < v1; v += kRowT * V) {
     Vec<V> y;
     if (delta) {
-      if constexpr (CL > 1) {
-        y = slab_sum_vec<V>(delta + t * d + v, n_partials, partial_stride);
-      } else {      // a long launch's few slabs: other rows cover the reads, and slab_sum_vec's batch would mostly repeat the last
-        y = load_vec<V>(delta + t * d + v);
-        for (int s = 1; s < n_partials; ++s) y.add(load_vec<V>(delta + t * d + v + s * partial_stride));
-      }
+      y = slab_sum_vec<V>(delta + t * d + v, n_partials, partial_stride);
     } else {
 #pragma unroll
       for (int k = 0; k < V; ++k) y.x[k] = 0.f;
@@ -237,6 +232,102 @@ sandwich_row_kernel(float* residual, const float* delta, int n_partials, long lo
   if (mine && xn) store_vec<4>(xn + t * d + 4 * v, x);
 }
 
+// Prompts: a row per CTA, kept in registers; all reads of a thread are on their way before the first is used.  12,390 rows of 2048:
+// 91 -> 74 us (a row staged in shared memory before), 6,500 with eight experts' rows each 123 -> 103.
+template <typename T, int THREADS, int NV>
+__global__ void __launch_bounds__(THREADS)
+sandwich_long_kernel(float* residual, const float* delta, int n_partials, long long partial_stride, const float* __restrict__ w_post,
+                     const float* __restrict__ w_next, T* xn, int d, float eps, const NormExtra extra) {
+  __shared__ RowSum<THREADS, 1, 1> sh;
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long t = blockIdx.x;
+  const int nvec = d / 4;
+  Vec<4> x[NV], y[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int v = static_cast<int>(threadIdx.x) + j * THREADS;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[j].x[k] = y[j].x[k] = 0.f;
+    if (v < nvec) {
+      if (delta) y[j] = load_vec<4>(delta + t * d + 4 * v);
+      x[j] = load_vec<4>(residual + t * d + 4 * v);
+    }
+  }
+  for (int s = 1; s < (delta ? n_partials : 0); ++s) {
+    Vec<4> p[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (static_cast<int>(threadIdx.x) + j * THREADS < nvec) p[j] = load_vec<4>(delta + t * d + 4 * (threadIdx.x + j * THREADS) + s * partial_stride);
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (static_cast<int>(threadIdx.x) + j * THREADS < nvec) y[j].add(p[j]);
+  }
+  if (extra.bias) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (static_cast<int>(threadIdx.x) + j * THREADS < nvec) y[j].add(load_vec<4>(extra.bias + 4 * (threadIdx.x + j * THREADS)));
+  }
+  for (int k = 0; k < extra.per_row; ++k) {
+    const float* row = extra.rows + static_cast<long long>(extra.index[t * extra.per_row + k]) * d;
+    const float f = extra.weight ? extra.weight[t * extra.per_row + k] : 1.0f;
+    Vec<4> p[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (static_cast<int>(threadIdx.x) + j * THREADS < nvec) p[j] = load_vec<4>(row + 4 * (threadIdx.x + j * THREADS));
+    for (int s = 1; s < extra.n_partials; ++s)
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+        if (static_cast<int>(threadIdx.x) + j * THREADS < nvec)
+          p[j].add(load_vec<4>(row + 4 * (threadIdx.x + j * THREADS) + s * extra.partial_stride));
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (static_cast<int>(threadIdx.x) + j * THREADS < nvec)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[j].x[i] = fmaf(f, p[j].x[i], y[j].x[i]);
+  }
+  const float inv_d = 1.0f / static_cast<float>(d);
+  float ss[1] = {0.f};
+  if (w_post) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) ss[0] += y[j].sumsq();
+    row_sum(sh, ss, 0);
+    const float inv = rsqrtf(ss[0] * inv_d + eps);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int v = static_cast<int>(threadIdx.x) + j * THREADS;
+      if (v < nvec) {
+        const Vec<4> w = load_vec<4>(w_post + 4 * v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[j].x[k] = fmaf(y[j].x[k], inv * w.x[k], x[j].x[k]);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) x[j].add(y[j]);
+  }
+  float inv = 1.0f;
+  if (w_next) {
+    ss[0] = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) ss[0] += x[j].sumsq();
+    row_sum(sh, ss, 1);
+    inv = rsqrtf(ss[0] * inv_d + eps);
+  }
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int v = static_cast<int>(threadIdx.x) + j * THREADS;
+    if (v >= nvec) break;
+    store_vec<4>(residual + t * d + 4 * v, x[j]);
+    if (w_next) {
+      const Vec<4> w = load_vec<4>(w_next + 4 * v);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[j].x[k] *= inv * w.x[k];
+    }
+    if (xn) store_vec<4>(xn + t * d + 4 * v, x[j]);
+  }
+}
+
 template <typename T, int V>
 __global__ void __launch_bounds__(kRowT)
 rows_norm_kernel(const float* __restrict__ residual, const int* __restrict__ rows, const float* __restrict__ w,
@@ -296,24 +387,25 @@ poly_norm_kernel(const float* __restrict__ z, int n_partials, long long partial_
   }
 }
 
-// A few rows, NV vectors per thread, kept in registers between the sums and the polynomial.  Eight rows of 7424 in a
-// captured step: 7.2 -> 5.4 us.
-template <typename T, int NV>
+// NV vectors per thread, kept in registers between the sums and the polynomial: a few rows over clusters (eight of 7424 in a captured
+// step: 7.2 -> 5.4 us), or prompts with a CTA per row (12,390 of 7424: 127 -> 106 us).
+template <typename T, int NV, int CL>
 __global__ void __launch_bounds__(kRowT)
 poly_row_kernel(const float* z, int n_partials, long long partial_stride, const float* __restrict__ coef, T* out, int ff, float eps) {
-  constexpr int CL = kRowCluster;
   __shared__ RowSum<kRowT, CL, 3> sh;
   pdl_launch_dependents();
   row_sum_begin(sh);
   const float c0 = coef[0], c1 = coef[1], c2 = coef[2], e = coef[3];
-  const int per = (ff / 4 + CL - 1) / CL, v0 = static_cast<int>(blockIdx.x) * per, v1 = min(ff / 4, v0 + per);
-  const long long t = blockIdx.y;
+  const int per = (ff / 4 + CL - 1) / CL, v0 = CL > 1 ? static_cast<int>(blockIdx.x) * per : 0, v1 = min(ff / 4, v0 + per);
+  const long long t = CL > 1 ? blockIdx.y : blockIdx.x;
   pdl_wait();
   Vec<4> x[NV];
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
     const int v = v0 + static_cast<int>(threadIdx.x) + j * kRowT;
-    x[j] = slab_sum_vec<4>(z + t * ff + 4 * min(v, ff / 4 - 1), n_partials, partial_stride);
+    const float* src = z + t * ff + 4 * min(v, ff / 4 - 1);
+    if constexpr (CL > 1) x[j] = slab_sum_vec<4>(src, n_partials, partial_stride);
+    else x[j] = load_vec<4>(src);
     if (v >= v1)
 #pragma unroll
       for (int k = 0; k < 4; ++k) x[j].x[k] = 0.f;
@@ -395,6 +487,10 @@ static int sandwich_t(float* residual, const float* delta, int n_partials, long 
   } else if (cl) {
     BCG_CUDA_CHECK(launch_cluster(sandwich_norm_kernel<T, V, kRowCluster>, dim3(kRowCluster, T_rows), dim3(kRowT),
                                   kRowCluster, sm, st, residual, delta, n_partials, stride, w_post, w_next, x, d, eps, extra));
+  } else if (V == 4 && T_rows > kClusterMaxRows && d <= 8192) {
+    const auto kernel = d <= 2048 ? sandwich_long_kernel<T, 128, 4> : d <= 4096 ? sandwich_long_kernel<T, 256, 4> : sandwich_long_kernel<T, 256, 8>;
+    BCG_CUDA_CHECK(launch_k(kernel, dim3(T_rows), dim3(d <= 2048 ? 128 : 256), 0, st, residual, delta, n_partials, stride, w_post, w_next, x,
+                            d, eps, extra));
   } else {
     BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(sandwich_norm_kernel<T, V, 1>), 200 * 1024));
     BCG_CUDA_CHECK(launch_k(sandwich_norm_kernel<T, V, 1>, dim3(T_rows), dim3(kRowT), sm, st, residual, delta, n_partials,
@@ -421,11 +517,14 @@ static int poly_t(const float* z, int n_partials, long long stride, const float*
   T* o = static_cast<T*>(out);
   const int vecs = (ff / 4 + kRowCluster - 1) / kRowCluster;     // of a CTA
   if (cl && V == 4 && vecs <= 2 * kRowT) {
-    const auto kernel = vecs <= kRowT ? poly_row_kernel<T, 1> : poly_row_kernel<T, 2>;
+    const auto kernel = vecs <= kRowT ? poly_row_kernel<T, 1, kRowCluster> : poly_row_kernel<T, 2, kRowCluster>;
     BCG_CUDA_CHECK(launch_cluster(kernel, dim3(kRowCluster, T_rows), dim3(kRowT), kRowCluster, 0, st, z, n_partials, stride, coef, o, ff, eps));
   } else if (cl) {
     BCG_CUDA_CHECK(launch_cluster(poly_norm_kernel<T, V, kRowCluster>, dim3(kRowCluster, T_rows), dim3(kRowT), kRowCluster,
                                   sm, st, z, n_partials, stride, coef, o, ff, eps));
+  } else if (V == 4 && T_rows > kClusterMaxRows && n_partials == 1 && ff <= 16 * 4 * kRowT) {
+    const auto kernel = ff <= 4 * 4 * kRowT ? poly_row_kernel<T, 4, 1> : ff <= 8 * 4 * kRowT ? poly_row_kernel<T, 8, 1> : poly_row_kernel<T, 16, 1>;
+    BCG_CUDA_CHECK(launch_k(kernel, dim3(T_rows), dim3(kRowT), 0, st, z, n_partials, stride, coef, o, ff, eps));
   } else {
     BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(poly_norm_kernel<T, V, 1>), 200 * 1024));
     BCG_CUDA_CHECK(launch_k(poly_norm_kernel<T, V, 1>, dim3(T_rows), dim3(kRowT), sm, st, z, n_partials, stride, coef, o,

@@ -363,3 +363,16 @@ def test_gemm_any_keeps_infinities_and_nans():
         assert torch.equal(out.isnan().cpu(), want.isnan()) and torch.equal(out.isinf().cpu(), want.isinf())
         ok = want.isfinite()
         torch.testing.assert_close(out.cpu()[ok], want[ok], rtol=1e-5, atol=1e-4)
+
+
+# Long launches keep a row in registers: the widest row of each form, ragged ends, several slabs, and the next width.
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("T,d,parts", [(129, 2048, 3), (140, 2052, 1), (129, 4096, 2), (131, 8192, 1), (129, 8196, 2), (150, 4, 1)])
+def test_sandwich_norm_of_long_launches(dtype, T, d, parts):
+    test_sandwich_norm(dtype, T, d, parts)
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("T,ff,parts", [(129, 4096, 1), (130, 7424, 1), (129, 16384, 1), (129, 16388, 1), (129, 4100, 2)])
+def test_poly_norm_of_long_launches(dtype, T, ff, parts):
+    test_poly_norm(dtype, T, ff, parts)
