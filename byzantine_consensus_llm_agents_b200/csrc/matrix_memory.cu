@@ -542,7 +542,7 @@ template <typename T, int NP>
 static int run_np(const MemArgs& a, int n_seqs, bool stream, bool chunks, cudaStream_t st) {
   const dim3 grid(a.heads, a.blocks(), n_seqs);
   if (stream) return launch_stream<T, NP>(a, n_seqs, st);
-  if (chunks) return launch_chunks<(NP < 64 ? 64 : NP), MemoryRule>(a, grid, st);
+  if (chunks) return launch_chunks<(NP < 64 ? 64 : NP), MemoryRule>(a, grid, a.n_tokens, n_seqs, st);
   BCG_CUDA_CHECK(launch_k(memory_scan_kernel<T, NP>, grid, dim3(kSsThreads), 0, st, a));
   return BCG_OK;
 }

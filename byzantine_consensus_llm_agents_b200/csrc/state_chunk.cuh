@@ -115,17 +115,23 @@ __device__ __forceinline__ void chunk_matrix(const RULE& rule, uint32_t sB, uint
   }
 }
 
-// grid (heads, blocks of 64 head entries, sequences); warp w has entries 16 w .. 16 w + 15 of the block.
-template <int NP, class RULE>
+// grid (heads * SEG, blocks of 64 head entries, sequences); warp w has entries 16 w .. 16 w + 15 of the block.
+//
+// SEG > 1 (rules without normalizer): few heads and sequences leave most of the chip idle while each walks its chunks one by one.
+// A cluster of SEG CTAs then shares a sequence's chunks: each first runs its part's state alone, from zero (a state's update, less
+// than half of a chunk's work), the states are handed on from CTA to CTA, S <- (what the part adds) + (its decay) S, and with the
+// state that comes in each runs its part whole.  64 heads, launches of 2,048 and of 951 tokens: 116 -> 63 us on average.
+template <int NP, class RULE, int SEG>
 __global__ void __launch_bounds__(kChThreads, ChCfg<NP, RULE>::kCtasPerSm)
 chunk_kernel(const typename RULE::Args a) {
+  static_assert(SEG == 1 || !RULE::kNormalized, "the normalizer is not handed on");
   using C = ChCfg<NP, RULE>;
   extern __shared__ __align__(128) uint8_t ch_raw[];
   const uint32_t base = (smem_u32(ch_raw) + 127u) & ~127u;
   float* scalars = reinterpret_cast<float*>(ch_raw + (base - smem_u32(ch_raw)) + C::kOffS);     // [2][kScalars]
   const uint32_t sC = base + C::kOffC, sM = base + C::kOffM, sN = base + C::kOffN;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.x, p0 = blockIdx.y * kSsRows, sq = blockIdx.z;
+  const int h = blockIdx.x / SEG, seg = blockIdx.x % SEG, p0 = blockIdx.y * kSsRows, sq = blockIdx.z;
   const int rows = min(kSsRows, a.vdim - p0), N = a.entries(), inner = a.inner();
   const bool normalizer = RULE::kNormalized && blockIdx.y == 0;
   pdl_launch_dependents();
@@ -158,19 +164,18 @@ chunk_kernel(const typename RULE::Args a) {
   const int q2 = (lane & 3) * 2;
   float* head = a.state_of(a.state_slots[sq], h);
   float* st = head + static_cast<long long>(p0) * N;
-  copy_rows(BCUnits{}, base, b_col, N, t0);
-  copy_rows(BCUnits{}, sC, c_col, N, t0);
-  copy_rows(XUnits{}, base + C::kOffX, x_col, rows, t0);
-  cp_async_commit();
+  const int c0 = SEG > 1 ? seg * n_chunks / SEG : 0, c1 = SEG > 1 ? (seg + 1) * n_chunks / SEG : n_chunks;     // this CTA's chunks
   float S[NP / 8][4];
   const bool fresh = a.positions[t0] == 0;
+  auto load_state = [&](bool zero) {
 #pragma unroll
-  for (int nt = 0; nt < NP / 8; ++nt)
+    for (int nt = 0; nt < NP / 8; ++nt)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int p = pr + (i >> 1) * 8, n = nt * 8 + q2 + (i & 1);
-      S[nt][i] = !fresh && p < rows && n < N ? st[static_cast<long long>(p) * N + n] : 0.f;
-    }
+      for (int i = 0; i < 4; ++i) {
+        const int p = pr + (i >> 1) * 8, n = nt * 8 + q2 + (i & 1);
+        S[nt][i] = !zero && p < rows && n < N ? st[static_cast<long long>(p) * N + n] : 0.f;
+      }
+  };
   // warp 0: the scalars of chunk c, then what those of the chunk behind it are made of
   RULE rule(a, h, t0, t1, static_cast<int>(blockIdx.y), fresh);
   const float skip = rule.skip();
@@ -178,10 +183,129 @@ chunk_kernel(const typename RULE::Args a) {
     rule.scalars(scalars + (c & 1) * RULE::kScalars, c, lane);
     rule.request(c + 1, lane);
   };
-  if (warp == 0) {
-    rule.request(0, lane);
-    scalars_of(0);
+  auto start_scalars = [&]() {
+    if (warp == 0) {
+      rule.request(c0, lane);
+      scalars_of(c0);
+    }
+  };
+  // hi and lo halves of w x for tokens 16 jp .. of the chunk; xf: x itself
+  auto weigh = [&](const float* w_s, int jp, const uint32_t (&xa)[4], float (&xf)[4][2], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      xf[i][0] = bf16lo(xa[i]);
+      xf[i][1] = bf16hi(xa[i]);
+    }
+    const float2 w0 = *reinterpret_cast<const float2*>(w_s + jp * 16 + q2), w1 = *reinterpret_cast<const float2*>(w_s + jp * 16 + 8 + q2);
+    split_bf16(w0.x * xf[0][0], w0.y * xf[0][1], hi[0], lo[0]);
+    split_bf16(w0.x * xf[1][0], w0.y * xf[1][1], hi[1], lo[1]);
+    split_bf16(w1.x * xf[2][0], w1.y * xf[2][1], hi[2], lo[2]);
+    split_bf16(w1.x * xf[3][0], w1.y * xf[3][1], hi[3], lo[3]);
+  };
+  const uint32_t r8 = (lane & 7) + ((lane >> 4) << 3), x8 = (((lane >> 3) & 1) ^ (lane & 7)) << 4;
+  // S^T += (w x)^T B of tokens 16 jp ..
+  auto advance = [&](uint32_t sB, int jp, const uint32_t (&hi)[4], const uint32_t (&lo)[4]) {
+    const uint32_t pb = sB + (lane & 15) * NP * 2, xb = ((lane >> 4) ^ (lane & 7)) << 4;
+#pragma unroll
+    for (int np = 0; np < NP / 16; np += 2) {
+      uint32_t b0[4], b1[4];
+      ldsm_trans_at(b0, pb + (xb ^ (np << 5)) + jp * 16 * NP * 2);
+      ldsm_trans_at(b1, pb + (xb ^ ((np + 1) << 5)) + jp * 16 * NP * 2);
+      mma_bf16_16816(S[2 * np], hi, b0[0], b0[1]);
+      mma_bf16_16816(S[2 * np + 1], hi, b0[2], b0[3]);
+      mma_bf16_16816(S[2 * np + 2], hi, b1[0], b1[1]);
+      mma_bf16_16816(S[2 * np + 3], hi, b1[2], b1[3]);
+      mma_bf16_16816(S[2 * np], lo, b0[0], b0[1]);
+      mma_bf16_16816(S[2 * np + 1], lo, b0[2], b0[3]);
+      mma_bf16_16816(S[2 * np + 2], lo, b1[0], b1[1]);
+      mma_bf16_16816(S[2 * np + 3], lo, b1[2], b1[3]);
+    }
+  };
+  auto decay = [&](float keep) {
+#pragma unroll
+    for (int nt = 0; nt < NP / 8; ++nt) {
+      scale2(S[nt][0], S[nt][1], keep, keep);
+      scale2(S[nt][2], S[nt][3], keep, keep);
+    }
+  };
+  if constexpr (SEG > 1) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    // ---- what the part adds to the state, and its decay
+    auto copy_inputs = [&](int c) {
+      copy_rows(BCUnits{}, base + (c & 1) * C::kBC, b_col, N, t0 + c * kChTok);
+      copy_rows(XUnits{}, base + C::kOffX + (c & 1) * C::kX, x_col, rows, t0 + c * kChTok);
+    };
+    load_state(fresh || seg > 0);
+    float total = 1.f;
+    if (c0 < c1 && seg + 1 < SEG) {
+      copy_inputs(c0);
+      cp_async_commit();
+      start_scalars();
+      for (int c = c0; c < c1; ++c) {
+        cp_async_wait<0>();
+        __syncthreads();
+        if (c + 1 < c1) copy_inputs(c + 1);
+        cp_async_commit();
+        const float* sc = scalars + (c & 1) * RULE::kScalars;
+        if (warp == 0) scalars_of(c + 1);
+        const float keep = rule.keep(sc);
+        total *= keep;
+        decay(keep);
+        const uint32_t px = base + C::kOffX + (c & 1) * C::kX + r8 * kSsRows * 2 + (x8 ^ (warp << 5));
+#pragma unroll
+        for (int jp = 0; jp < kChTok / 16; ++jp) {
+          uint32_t xa[4], hi[4], lo[4];
+          float xf[4][2];
+          ldsm_trans_at(xa, px + jp * 16 * kSsRows * 2);
+          weigh(sc + 3 * kChTok, jp, xa, xf, hi, lo);
+          advance(base + (c & 1) * C::kBC, jp, hi, lo);
+        }
+      }
+    }
+    // ---- handed on through the place of B, which nobody reads now: a thread's entries are its successor's
+    float4* box = reinterpret_cast<float4*>(ch_raw + (base - smem_u32(ch_raw)));
+    cluster.sync();
+    for (int k = 0; k + 1 < SEG; ++k) {
+      if (seg == k) {
+        float4* dst = cluster.map_shared_rank(box, k + 1);
+#pragma unroll
+        for (int nt = 0; nt < NP / 8; ++nt) dst[nt * kChThreads + threadIdx.x] = make_float4(S[nt][0], S[nt][1], S[nt][2], S[nt][3]);
+        if (k == 0) load_state(fresh);      // before the last CTA can write it
+      }
+      cluster.sync();
+      if (seg == k + 1) {
+#pragma unroll
+        for (int nt = 0; nt < NP / 8; ++nt) {
+          const float4 v = box[nt * kChThreads + threadIdx.x];
+          if (k + 2 < SEG) {
+            S[nt][0] = fmaf(total, v.x, S[nt][0]);
+            S[nt][1] = fmaf(total, v.y, S[nt][1]);
+            S[nt][2] = fmaf(total, v.z, S[nt][2]);
+            S[nt][3] = fmaf(total, v.w, S[nt][3]);
+          }
+        }
+      }
+    }
+    if (seg > 0) {
+#pragma unroll
+      for (int nt = 0; nt < NP / 8; ++nt) {
+        const float4 v = box[nt * kChThreads + threadIdx.x];
+        S[nt][0] = v.x;
+        S[nt][1] = v.y;
+        S[nt][2] = v.z;
+        S[nt][3] = v.w;
+      }
+    }
+    if (c0 >= c1) return;
+    __syncthreads();
   }
+  copy_rows(BCUnits{}, base + (c0 & 1) * C::kBC, b_col, N, t0 + c0 * kChTok);
+  copy_rows(BCUnits{}, sC, c_col, N, t0 + c0 * kChTok);
+  copy_rows(XUnits{}, base + C::kOffX + (c0 & 1) * C::kX, x_col, rows, t0 + c0 * kChTok);
+  cp_async_commit();
+  if constexpr (SEG == 1) load_state(fresh);
+  start_scalars();
   // normalizer: a thread has entries e0 .. of it, and writes them as two halves for the products
   constexpr int kPer = NP / kChThreads > 0 ? NP / kChThreads : 1;
   const int e0 = static_cast<int>(threadIdx.x) * kPer;
@@ -203,14 +327,14 @@ chunk_kernel(const typename RULE::Args a) {
     }
   }
 
-  for (int c = 0; c < n_chunks; ++c) {
+  for (int c = c0; c < c1; ++c) {
     const int first = t0 + c * kChTok, nt_tok = min(kChTok, t1 - first);
     const float* sc = scalars + (c & 1) * RULE::kScalars;
     const float* w_s = sc + 3 * kChTok;
     cp_async_wait<0>();
     __syncthreads();                            // the chunk is there, everybody is done with the previous one
     const uint32_t sB = base + (c & 1) * C::kBC, sX = base + C::kOffX + (c & 1) * C::kX;
-    if (c + 1 < n_chunks) {
+    if (c + 1 < c1) {
       copy_rows(BCUnits{}, base + ((c + 1) & 1) * C::kBC, b_col, N, first + kChTok);
       copy_rows(XUnits{}, base + C::kOffX + ((c + 1) & 1) * C::kX, x_col, rows, first + kChTok);
     }
@@ -225,7 +349,6 @@ chunk_kernel(const typename RULE::Args a) {
 
     // ---- Y^T = S^T C^T, columns (tokens) scaled by exp(c_i)
     float Y[kChTok / 8][4] = {};
-    const uint32_t r8 = (lane & 7) + ((lane >> 4) << 3), x8 = (((lane >> 3) & 1) ^ (lane & 7)) << 4;
     const uint32_t pc = sC + r8 * NP * 2;
 #pragma unroll
     for (int k = 0; k < NP / 16; ++k) {
@@ -246,13 +369,9 @@ chunk_kernel(const typename RULE::Args a) {
       scale2(Y[it][2], Y[it][3], e.x, e.y);
     }
     const float keep = rule.keep(sc);
-#pragma unroll
-    for (int nt = 0; nt < NP / 8; ++nt) {
-      scale2(S[nt][0], S[nt][1], keep, keep);
-      scale2(S[nt][2], S[nt][3], keep, keep);
-    }
+    decay(keep);
     __syncthreads();                            // M is complete, C has been read
-    if (c + 1 < n_chunks) copy_rows(BCUnits{}, sC, c_col, N, first + kChTok);
+    if (c + 1 < c1) copy_rows(BCUnits{}, sC, c_col, N, first + kChTok);
     cp_async_commit();
     if constexpr (RULE::kNormalized) {
       if (normalizer && e0 < NP) {
@@ -280,7 +399,6 @@ chunk_kernel(const typename RULE::Args a) {
 
     // ---- Y^T += x^T M^T + skip x^T;   S^T += (w x)^T B
     const uint32_t px = sX + r8 * kSsRows * 2 + (x8 ^ (warp << 5));
-    const uint32_t pb = sB + (lane & 15) * NP * 2, xb = ((lane >> 4) ^ (lane & 7)) << 4;
     const uint32_t pm = sM + r8 * kChTok * 2;
 #pragma unroll
     for (int jp = 0; jp < kChTok / 16; ++jp) {
@@ -295,11 +413,8 @@ chunk_kernel(const typename RULE::Args a) {
           mma_bf16_16816(Y[2 * ip + 1], xa, mb[2], mb[3]);
         }
       float xf[4][2];                           // rows pr, pr + 8 of tokens j, j + 1; the same of tokens j + 8, j + 9
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        xf[i][0] = bf16lo(xa[i]);
-        xf[i][1] = bf16hi(xa[i]);
-      }
+      uint32_t hi[4], lo[4];
+      weigh(w_s, jp, xa, xf, hi, lo);
       if constexpr (!RULE::kNormalized) {
 #pragma unroll
         for (int e = 0; e < 2; ++e)
@@ -309,26 +424,7 @@ chunk_kernel(const typename RULE::Args a) {
             Y[2 * jp + e][2 + k] = fmaf(skip, xf[2 * e + 1][k], Y[2 * jp + e][2 + k]);
           }
       }
-      const float2 w0 = *reinterpret_cast<const float2*>(w_s + jp * 16 + q2), w1 = *reinterpret_cast<const float2*>(w_s + jp * 16 + 8 + q2);
-      uint32_t hi[4], lo[4];
-      split_bf16(w0.x * xf[0][0], w0.y * xf[0][1], hi[0], lo[0]);
-      split_bf16(w0.x * xf[1][0], w0.y * xf[1][1], hi[1], lo[1]);
-      split_bf16(w1.x * xf[2][0], w1.y * xf[2][1], hi[2], lo[2]);
-      split_bf16(w1.x * xf[3][0], w1.y * xf[3][1], hi[3], lo[3]);
-#pragma unroll
-      for (int np = 0; np < NP / 16; np += 2) {
-        uint32_t b0[4], b1[4];
-        ldsm_trans_at(b0, pb + (xb ^ (np << 5)) + jp * 16 * NP * 2);
-        ldsm_trans_at(b1, pb + (xb ^ ((np + 1) << 5)) + jp * 16 * NP * 2);
-        mma_bf16_16816(S[2 * np], hi, b0[0], b0[1]);
-        mma_bf16_16816(S[2 * np + 1], hi, b0[2], b0[3]);
-        mma_bf16_16816(S[2 * np + 2], hi, b1[0], b1[1]);
-        mma_bf16_16816(S[2 * np + 3], hi, b1[2], b1[3]);
-        mma_bf16_16816(S[2 * np], lo, b0[0], b0[1]);
-        mma_bf16_16816(S[2 * np + 1], lo, b0[2], b0[3]);
-        mma_bf16_16816(S[2 * np + 2], lo, b1[0], b1[1]);
-        mma_bf16_16816(S[2 * np + 3], lo, b1[2], b1[3]);
-      }
+      advance(sB, jp, hi, lo);
     }
 
     // ---- store: pairs are transposed on the way out (token lane >> 2, entries q2, q2 + 1)
@@ -354,6 +450,7 @@ chunk_kernel(const typename RULE::Args a) {
       out += 8ll * inner;
     }
   }
+  if (c1 < n_chunks) return;
 #pragma unroll
   for (int nt = 0; nt < NP / 8; ++nt)
 #pragma unroll
@@ -371,13 +468,29 @@ chunk_kernel(const typename RULE::Args a) {
   rule.finish(sq, p0, rows, fresh);
 }
 
-template <int NP, class RULE>
-static int launch_chunks(const typename RULE::Args& a, dim3 grid, cudaStream_t st) {
+template <int NP, class RULE, int SEG>
+static int launch_segments(const typename RULE::Args& a, dim3 grid, cudaStream_t st) {
   constexpr int kSmem = ChCfg<NP, RULE>::kSmem;
-  BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(chunk_kernel<NP, RULE>), kSmem));
-  BCG_CUDA_CHECK(launch_k(chunk_kernel<NP, RULE>, grid, dim3(kChThreads), kSmem, st, a));
+  const auto kernel = chunk_kernel<NP, RULE, SEG>;
+  BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kSmem));
+  grid.x *= SEG;
+  if constexpr (SEG == 1) {
+    BCG_CUDA_CHECK(launch_k(kernel, grid, dim3(kChThreads), kSmem, st, a));
+  } else {
+    BCG_CUDA_CHECK(launch_cluster(kernel, grid, dim3(kChThreads), SEG, kSmem, st, a));
+  }
   return BCG_OK;
 }
-
+// n_tokens of n_seqs sequences, whose lengths only the device knows.  Parts while their CTAs have a slot and two chunks each.
+template <int NP, class RULE>
+static int launch_chunks(const typename RULE::Args& a, dim3 grid, int n_tokens, int n_seqs, cudaStream_t st) {
+  if constexpr (!RULE::kNormalized) {
+    const long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z, slots = 148ll * ChCfg<NP, RULE>::kCtasPerSm;
+    const int chunks = n_tokens / n_seqs / kChTok;
+    if (ctas * 4 <= slots && chunks >= 8) return launch_segments<NP, RULE, 4>(a, grid, st);
+    if (ctas * 2 <= slots && chunks >= 4) return launch_segments<NP, RULE, 2>(a, grid, st);
+  }
+  return launch_segments<NP, RULE, 1>(a, grid, st);
+}
 
 }  // namespace bcg

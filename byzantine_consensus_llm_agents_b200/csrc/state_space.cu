@@ -743,7 +743,7 @@ static int run_np(const SsmArgs& a, int n_seqs, bool one_token, bool chunks, cud
     BCG_CUDA_CHECK(launch_k(ssm_token_kernel<T, NP>, grid, dim3(kSsThreads), 0, st, a));
   } else if (chunks) {
     constexpr int P = NP < 64 ? 64 : NP;
-    BCG_TRY((launch_chunks<P, SsdRule>(a, grid, st)));
+    BCG_TRY((launch_chunks<P, SsdRule>(a, grid, a.n_tokens, n_seqs, st)));
   } else {
     BCG_CUDA_CHECK(launch_k(ssm_scan_kernel<T, NP>, grid, dim3(kSsThreads), 0, st, a));
   }

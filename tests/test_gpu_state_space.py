@@ -428,3 +428,27 @@ def test_embedding_with_sinusoids_at_far_positions(width):
     want = a.t["embed"][:7].double() * 3.0 + R.sinusoid(torch.tensor(pos), width)
     assert (a.get("residual", 7, width).double() - want).abs().max() < 2e-6
     close(a.get("xn", 7, width), R.zero_norm(want, 1e-5, a.t["final.norm"].double()), 2e-6)
+
+
+@pytest.mark.parametrize("size", ["usual", "blocks", "wide", "odd", "halves", "one", "many"])
+def test_long_sequences_in_parts(size):
+    """Four and two CTAs share a sequence's chunks: lengths at and off chunk ends, continued from a state, beside sequences that have
+    fewer chunks than there are parts.  Sums in another order than token by token, the same roundings of operands."""
+    a = StateSpace(size, "bfloat16", kv_pages=256, max_model_len=1024)
+    proj = {s: _proj(a, n, s) for s, n in enumerate((1000, 513, 2, 70))}
+    want = {s: a.oracle(p) for s, p in proj.items()}
+    for sizes in ([1000], [512, 488], [333, 600, 67]):
+        a.junk()
+        a.check(a.feed(proj[0], sizes, 0), want[0][0], a.tol)
+        close(a.state[0], want[0][1], a.tol)
+        if a.m["conv"] > 1:
+            close(a.conv[0], want[0][2], 1e-5)
+    a.junk()
+    untouched = a.state[5].clone()
+    for group in ([1, 2], [3, 1]):      # 257 and 291 tokens per sequence
+        out = a.run([(len(proj[s]), 0, s) for s in group], torch.cat([proj[s] for s in group]))
+        for s in group:
+            a.check(out[:len(proj[s])], want[s][0], a.tol)
+            out = out[len(proj[s]):]
+            close(a.state[s], want[s][1], a.tol)
+    assert torch.equal(a.state[5], untouched)
