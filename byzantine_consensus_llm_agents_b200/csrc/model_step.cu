@@ -57,15 +57,13 @@ int model_prefill(const bcg_model* m, const bcg_workspace* ws, const int* ids, c
     set_last_error("bcg_model_prefill", "tp_size does not match bcg_tp_init");
     return BCG_ERR_ARG;
   }
-  // slabs of the products whose consumer is the norm: the all-reduce between them and the head, which comes back to the last
-  // layer's product for other rows, take one
-  const long long room = static_cast<long long>(ws->T_max) * d;
-  const int s_o = tp > 1 ? 1 : gemm_long_splits(T, d, hq * 128, room), s_dn = tp > 1 ? 1 : gemm_long_splits(T, d, m->d_ff, room);
+  // Products are never cut along K here: the best number of parts depends on the launch's rows, and a prompt's logits and cached
+  // pages must not depend on what else is in the launch.  It has a price: 256 x 12288 -> 4096 takes 65.7 us whole, 31.4 in four parts.
   for (int l = 0; l < m->n_layers; ++l) {
     if (l == 0) {
       BCG_TRY(embed_rmsnorm(ids, m->embed, m->ln1[0], ws->residual, ws->xn, T, d, m->rms_eps, st));
     } else {
-      BCG_TRY(add_rmsnorm(ws->residual, ws->delta, 1, s_dn, static_cast<long long>(T) * d, m->ln1[l], ws->xn, nullptr, T, d,
+      BCG_TRY(add_rmsnorm(ws->residual, ws->delta, 1, 1, 0, m->ln1[l], ws->xn, nullptr, T, d,
                           m->rms_eps, st));
     }
     // projections that feed fp32 consumers keep their fp32 accumulators (no bf16 round trip)
@@ -77,14 +75,14 @@ int model_prefill(const bcg_model* m, const bcg_workspace* ws, const int* ids, c
     BCG_TRY(prefill_attn_paged(ws->q, m->kv_cache[l], block_table, max_blocks, tile_info, n_tiles,
                                ws->attn, T, hq, hkv, m->page_size, scale, st));
     BCG_TRY(gemm_bf16_tn(ws->attn, m->w_o[l], ws->delta, T, d, hq * 128, hq * 128, hq * 128, d,
-                         BCG_EPI_F32, s_o, 0, st));
+                         BCG_EPI_F32, 1, 0, st));
     if (tp > 1) BCG_TRY(tp_all_reduce_f32(ws->delta, static_cast<long long>(T) * d, st));
-    BCG_TRY(add_rmsnorm(ws->residual, ws->delta, 1, s_o, static_cast<long long>(T) * d, m->ln2[l], ws->xn, nullptr, T, d,
+    BCG_TRY(add_rmsnorm(ws->residual, ws->delta, 1, 1, 0, m->ln2[l], ws->xn, nullptr, T, d,
                         m->rms_eps, st));
     BCG_TRY(gemm_bf16_tn(ws->xn, m->w_gate_up[l], ws->act, T, 2 * m->d_ff, d, d, d, m->d_ff,
                          BCG_EPI_SWIGLU, 1, 0, st));
     BCG_TRY(gemm_bf16_tn(ws->act, m->w_down[l], ws->delta, T, d, m->d_ff, m->d_ff, m->d_ff, d,
-                         BCG_EPI_F32, l + 1 < m->n_layers ? s_dn : 1, 0, st));
+                         BCG_EPI_F32, 1, 0, st));
     if (tp > 1) BCG_TRY(tp_all_reduce_f32(ws->delta, static_cast<long long>(T) * d, st));
   }
   return model_head(m, ws, last_rows, n_seqs, 0, st);

@@ -267,6 +267,26 @@ def test_waves_and_prefill_groups_do_not_change_results():
     assert all(r.prompt_tokens == n for r, n in zip(together, lens))
 
 
+@pytest.mark.parametrize("n", [60, 129, 200, 300, 513])
+def test_prompt_logits_do_not_depend_on_the_launch(n):
+    """A prompt's logits, and those of the tokens behind it (its cached pages), are the same bits alone, beside other prompts and in
+    an engine with another workspace: products of prompts sum over K in one order, whatever the launch's rows."""
+    w = Weights.random_init(WIDE_QWEN, torch.device("cuda:0"))
+    tk = get_tokenizer(WIDE_QWEN.family, WIDE_QWEN.vocab)
+    rng = np.random.default_rng(n)
+    prompts = _prompts(tk, rng, [n, 333, 64, 900])
+    forced = [rng.integers(*tk.regular_range, size=4).tolist() for _ in prompts]
+    got = []
+    for tokens, rows in ((1024, 1), (4096, 1), (4096, 2), (4096, 4)):
+        eng = Engine(WIDE_QWEN, w, tk, max_model_len=1024, max_rows=4, prefill_tokens=tokens, kv_pages=300, enable_prefix_cache=False)
+        eng.debug_logits = []
+        eng.generate([Request("", None, 0.0, 4, forced=f, prompt_ids=p) for p, f in zip(prompts[:rows], forced)])
+        got.append(torch.stack([x[0] for x in eng.debug_logits]))
+        eng.close()
+    for other in got[1:]:
+        assert torch.equal(got[0], other)
+
+
 @pytest.mark.parametrize("preset,n_layers,lens", [("qwen3-14b", 4, [520, 77]), ("qwen3-8b", 2, [520, 77]),
                                                   ("qwen3-32b", 2, [520, 77]), ("mistral-22b", 2, [600, 77])])
 def test_full_width_reduced_depth_logits(preset, n_layers, lens):
