@@ -393,22 +393,6 @@ struct DsCfg {
   static constexpr int kFloats = 2 * kChunk * kOps + 2 * kChunk * kCols + kChunk * 6 * DP;
 };
 
-// wait for a cluster-wide phase; a phase that never comes traps instead of hanging
-__device__ __forceinline__ void mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok = 0, spins = 0;
-  while (!ok) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.b32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (++spins > (1u << 26)) __trap();
-  }
-}
 __device__ __forceinline__ uint32_t peer_smem(const void* p, int rank) {
   uint32_t r;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));

@@ -154,7 +154,7 @@ __device__ __forceinline__ void row_sum(RowSum<THREADS, CL, N>& sh, float (&v)[N
             "r"(smem_u32(&sh.bar[slot & 1])), "r"(lane), "r"(__float_as_uint(v[k]))
             : "memory");
     }
-    mbar_wait(&sh.bar[slot & 1], 0);
+    mbar_wait_cluster(&sh.bar[slot & 1], 0);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       float t = 0.f;

@@ -237,3 +237,19 @@ def test_model_presets_reproduce_published_parameter_counts():
         assert abs(params(PRESETS[k]) - v) / v < 2e-3, (k, params(PRESETS[k]))
     assert abs(PRESETS["qwen3-14b"].decode_weight_bytes() - 27.98e9) < 0.02e9
     assert PRESETS["qwen3-14b"].kv_bytes_per_token == 163840
+
+
+def test_sums_from_other_ctas_are_waited_for_at_cluster_scope():
+    """Where peers of a cluster deliver with st.async or arrive remotely with plain stores in front, the reader's wait acquires at
+    cluster scope: a wait of CTA scope leaves its reads racing with the peers' stores (by the memory model, so read from the source)."""
+    found = 0
+    for path in sorted((ROOT / "byzantine_consensus_llm_agents_b200" / "csrc").glob("*.cu*")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for body in re.split(r"\n}\n", text):          # top-level definitions
+            if "st.async" in body:
+                found += 1
+                assert "mbar_wait_cluster(" in body, path.name
+                assert not re.search(r"\bmbar_(try_)?wait\(", body), path.name
+    assert found
+    wait = re.search(r"bool mbar_try_wait_cluster\(.*?\n}\n", (ROOT / "byzantine_consensus_llm_agents_b200/csrc/common.cuh").read_text(), re.S)
+    assert "acquire.cluster" in wait.group(0)
