@@ -1,6 +1,7 @@
 """The kernels of parallel layers one by one — grouped attention with a distance bias, its input split, experts,
 the residual addition, the squared-relu product — against the plain oracle (oracle/stack_ref.py)."""
 import ctypes as C
+import math
 
 import numpy as np
 import pytest
@@ -153,6 +154,28 @@ def test_grouped_attention_fp32_tiles(size, window):
     softmax average, so its error is a few units of fp32 times the scores' size, as with one token per CTA."""
     a = Attention(size, window, "float32")
     _check(a, _seqs(a, ((130, 33), (65, 64), (64, 1), (40, 3), (31, 31)), window), 3e-6)
+
+
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
+@pytest.mark.parametrize("window", [0, 17])
+def test_values_that_are_not_finite_reach_only_the_tokens_that_see_them(value, window):
+    """Two tokens of the second sequence have a value that is infinite or NaN; the first and third sequence share CTAs, and warps of
+    four queries, with it.  Whoever does not see them is exact as ever, and so are all other columns."""
+    a = Attention("usual", window, "float32")
+    seqs = _seqs(a, ((40, 21), (70, 34), (43, 43)), window)
+    odd = (45, 60)
+    for j in odd:
+        seqs[1][1][j, :, 3] = value
+    out, meta = a.run(seqs)
+    starts = np.cumsum([0] + [len(q) for _, _, q in seqs])
+    for t, (pos, k, v, q) in enumerate(meta):
+        reached = starts[1] <= t < starts[2] and any(max(0, pos - window + 1 if window else 0) <= j <= pos for j in odd)
+        want = a.oracle(pos, k, torch.nan_to_num(v, 0.0, 0.0, 0.0), q)
+        keep = [c for c in range(a.m["vdim"]) if c != 3 or not reached]
+        err = (out[t].double() - want)[:, keep].norm() / want[:, keep].norm()
+        assert err < 3e-6, (t, err.item())
+        if reached:
+            assert not torch.isfinite(out[t][:, 3]).any()
 
 
 @pytest.mark.parametrize("context", [1, 15, 16, 17, 333, 2000])
