@@ -1,8 +1,8 @@
 // out fp32 [M, ldo] = X fp32 [M, ldx] * W bf16 [N, ldw]^T with every product and sum of fp32 quality, on tensor cores.
 //
 // An fp32 number is the sum of three bf16 ones, cut off its top bits one after another (8 + 8 + 8 bits of mantissa, no rounding),
-// and the weights are bf16 already: X = X1 + X2 + X3, three bf16 products give every partial product exactly.  What is left to
-// rounding are the sums, and tensor cores cut what they add where FMAs round it: so only the 64 inputs of a k-block (smallest
+// and the weights are bf16 already: X = X1 + X2 + X3, three bf16 products give every partial product exactly (where |x| >= 2^-110 or
+// x = 0: below, the last parts leave bf16's range, an error of 2^-133 at most).  What is left to rounding are the sums, and tensor cores cut what they add where FMAs round it: so only the 64 inputs of a k-block (smallest
 // part first) meet in TMEM, and the blocks are added in registers.
 // Relative error against 64 bits (2-norm), one FMA chain per output / here: 8.1e-7 / 1.3e-7 at K = 2048, 1.9e-6 / 2.5e-7 at
 // K = 11264.
@@ -26,9 +26,10 @@ constexpr int split_smem(int bn) { return kSpStages * split_stage_bytes(bn) + 10
 
 struct SplitArgs {
   const float* x;
+  const __nv_bfloat16* w;
   float* out;
   int M, N, K, k_blocks, tiles_m;
-  long long ldx, ldo;
+  long long ldx, ldw, ldo;
   int vec_out;      // output rows start on 16 bytes
 };
 
@@ -38,9 +39,39 @@ __device__ __forceinline__ uint32_t top_halves(float a, float b) {
 }
 __device__ __forceinline__ float below_top(float a) { return a - __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
 
+// Outputs that came out as NaN, formed again by FMAs, by one warp: with parts, an infinite weight meets parts of x that are zero.  Rows
+// with a NaN among their activations keep theirs.  Covers the warp's own 32 rows and `cols` columns.  Looking for them costs nothing
+// that shows (820 x 2048 -> 12288: 208 us with and without).
+static __device__ __noinline__ void redo_nans(const SplitArgs& a, int m_first, int n_first, int cols) {
+  const int lane = threadIdx.x & 31;
+  for (int m = m_first; m < min(m_first + 32, a.M); ++m) {
+    const float* x = a.x + m * a.ldx;
+    bool settled = false;      // the row was looked at
+    for (int c0 = 0; c0 < cols; c0 += 32) {
+      const int n_lane = n_first + c0 + lane;
+      float* o = a.out + m * a.ldo + n_lane;
+      uint32_t left = __ballot_sync(0xffffffffu, c0 + lane < cols && n_lane < a.N && *o != *o);
+      if (left && !settled) {
+        bool nan = false;
+        for (int k = lane; k < a.K; k += 32) nan |= x[k] != x[k];
+        if (__any_sync(0xffffffffu, nan)) break;
+        settled = true;
+      }
+      for (; left; left &= left - 1) {
+        const int at = __ffs(left) - 1;
+        const __nv_bfloat16* w = a.w + (n_first + c0 + at) * a.ldw;
+        float s = 0.f;
+        for (int k = lane; k < a.K; k += 32) s = fmaf(x[k], __bfloat162float(w[k]), s);
+        s = warp_sum(s);
+        if (lane == at) *o = s;
+      }
+    }
+  }
+}
+
 template <int BN>
 __global__ void __launch_bounds__(kSpThreads, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const SplitArgs a) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ SplitArgs a) {
   constexpr int STAGE = split_stage_bytes(BN), W_BYTES = BN * kSpK * 2, COLS = BN / 2;
   constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
   constexpr uint32_t IDESC = make_idesc_bf16_m128(BN);
@@ -146,6 +177,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const SplitArgs a)
             if (n + c + j < a.N) o[c + j] = sum[c + j];
         }
       }
+    }
+    float odd = 0.f;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) odd = fmaf(0.f, sum[c], odd);
+    if (__any_sync(0xffffffffu, odd != 0.f && m < a.M)) {
+      __syncwarp();
+      redo_nans(a, m0 + q * 32, n, COLS);
     }
   } else {
     // eight lanes read 64 columns of a row, a warp four rows at a time
@@ -320,6 +358,7 @@ int gemm_f32(const float* X, const void* W, float* out, int M, int N, int K, lon
   }
   SplitArgs a = {};
   a.x = X;
+  a.w = static_cast<const __nv_bfloat16*>(W);
   a.out = out;
   a.M = M;
   a.N = N;
@@ -327,6 +366,7 @@ int gemm_f32(const float* X, const void* W, float* out, int M, int N, int K, lon
   a.k_blocks = (K + kSpK - 1) / kSpK;
   a.tiles_m = (M + kSpM - 1) / kSpM;
   a.ldx = ldx;
+  a.ldw = ldw;
   a.ldo = ldo;
   a.vec_out = (reinterpret_cast<uintptr_t>(out) % 16 == 0 && ldo % 4 == 0) ? 1 : 0;
   // Rounds of one CTA per SM; a narrow tile takes a little more than half the time of a wide one (the conversion is the same)

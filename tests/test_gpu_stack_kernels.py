@@ -1,5 +1,6 @@
 """The kernels of layer stacks one by one, against the plain oracle (oracle/stack_ref.py) on the same inputs."""
 import ctypes as C
+import math
 
 import numpy as np
 import pytest
@@ -363,6 +364,28 @@ def test_gemm_any_keeps_infinities_and_nans():
         assert torch.equal(out.isnan().cpu(), want.isnan()) and torch.equal(out.isinf().cpu(), want.isinf())
         ok = want.isfinite()
         torch.testing.assert_close(out.cpu()[ok], want[ok], rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("M", [1, 4, 5, 40, 300])
+@pytest.mark.parametrize("N,K", [(70, 512), (2500, 136)])
+def test_gemm_any_infinite_weights(M, N, K):
+    """An infinite weight gives what it gives in 64 bits, whatever the count of rows: infinity with the activation's sign, NaN where the
+    activation is zero (and where two infinities cancel), also where the activation has few bits and its lower parts are zero."""
+    g = gen(M)
+    x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g).bfloat16()
+    x[:, 7] = torch.tensor([1.0, -2.0, 0.0, 1.1])[torch.arange(M) % 4]
+    w[5, 7], w[33, 7], w[69, 7], w[64, 8], w[N - 1, K - 1] = math.inf, -math.inf, math.nan, math.inf, math.inf
+    w[12, 7], w[12, 8] = math.inf, math.inf
+    if M > 4:
+        x[4, 3] = math.nan
+    X, W = dev(x), dev(w)
+    out = torch.zeros(M, N, device="cuda")
+    L.check(L.load().bcg_gemm_any(X.data_ptr(), L.DT_F32, W.data_ptr(), out.data_ptr(), M, N, K, K, K, N, L.stream_ptr()))
+    want, got = (x.double() @ w.double().T).float(), out.cpu()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    ok = want.isfinite()
+    torch.testing.assert_close(got[ok], want[ok], rtol=1e-5, atol=1e-4)
 
 
 # Long launches keep a row in registers: the widest row of each form, ragged ends, several slabs, and the next width.
