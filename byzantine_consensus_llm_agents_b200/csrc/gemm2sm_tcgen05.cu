@@ -376,7 +376,8 @@ static bool for_pairs(int M, int N) {
 // clock and SM out of L2).  256 x 4096 -> 4096 in 1 / 2 / 4 parts: 29.8 / 21.5 / 17.8 us, 12288 -> 4096: 65.7 / 40.0 / 31.4; with
 // 951 rows 31.5 / 31.5 / 37.7 and 74.4 / 76.3 / 78.4, so that they stay whole.
 //
-// How many parts of K the fp32 product of a long launch is best cut into, where the consumer adds slabs: tiles that leave pairs of
+// How many parts of K the fp32 product of a long launch is best cut into, where the consumer adds slabs (in layer stacks; rows of
+// dense models must not depend on their launch): tiles that leave pairs of
 // SMs idle in the last round cost more than the slabs do.  Clocks: 520 per k-block and round (measured over 12 k rows; the MMAs
 // take 512), slabs written and read at about 4 KB per clock.  At most `room` floats of output.
 int gemm_long_splits(int M, int N, int K, long long room) {

@@ -24,10 +24,22 @@ static bool tensor_gemm(int act_dtype, int M, int N, int K) {
 int stack_splits(int act_dtype, int M, int N, int K) {
   return tensor_gemm(act_dtype, M, N, K) && M <= 128 ? gemm_splits_for(M, N, K) : 1;
 }
-// any_slabs: the consumer adds slabs in long launches too.
+// Columns of the widest product that leaves its output in ws->proj in a layer.
+static int widest(const bcg_layer* l) {
+  const bool paired = l->ff_kind == BCG_FF_CLAMPED_GLU || l->ff_kind == BCG_FF_GELU_GLU;
+  const int up = l->parallel ? 0 : l->ff_kind == BCG_FF_EXPERTS ? l->n_router + l->ff : paired ? 2 * l->ff : l->ff;
+  return l->n_in > up ? l->n_in : up;
+}
+// slabs: the consumer adds slabs in long launches too.  They take no more room than the layer's widest product, which the workspace
+// holds for as many rows: what fits must not depend on how many rows the workspace could hold.
 static int project(const bcg_stack* m, const void* x, const void* w, float* out, long long cap, int M, int N, int K,
-                   int* splits, cudaStream_t st, bool any_slabs = false) {
-  *splits = any_slabs && M > 128 && tensor_gemm(m->act_dtype, M, N, K) ? gemm_long_splits(M, N, K, cap) : stack_splits(m->act_dtype, M, N, K);
+                   int* splits, cudaStream_t st, const bcg_layer* slabs = nullptr) {
+  if (slabs && M > 128 && tensor_gemm(m->act_dtype, M, N, K)) {
+    const long long room = static_cast<long long>(M) * widest(slabs);
+    *splits = gemm_long_splits(M, N, K, room < cap ? room : cap);
+  } else {
+    *splits = stack_splits(m->act_dtype, M, N, K);
+  }
   if (static_cast<long long>(*splits) * M * N > cap) {
     set_last_error("bcg_stack_step", "projection scratch too small");
     return BCG_ERR_TOO_LARGE;
@@ -154,7 +166,7 @@ static int parallel_layer(const bcg_stack* m, const bcg_stack_ws* ws, const bcg_
     extra.partial_stride = static_cast<long long>(T) * l->top * d;
   }
   BCG_TRY(grouped_attention(m, ws, b, l, 0, st));
-  BCG_TRY(project(m, ws->mix, l->w_out, ws->proj, ws->proj_floats, T, d, l->mix_ld, &s, st, true));
+  BCG_TRY(project(m, ws->mix, l->w_out, ws->proj, ws->proj_floats, T, d, l->mix_ld, &s, st, l));
   return sandwich_norm(ws->residual, ws->proj, s, static_cast<long long>(T) * d, nullptr, next, ws->xn, dt, T, d, m->eps,
                        extra, st);
 }
@@ -191,7 +203,7 @@ static int expert_ff(const bcg_stack* m, const bcg_stack_ws* ws, const bcg_layer
   extra->per_row = l->top;
   extra->partial_stride = static_cast<long long>(T) * l->top * d;
   *splits = 0;
-  return l->ff > 0 ? project(m, ws->act, l->w_down, ws->proj, ws->proj_floats, T, d, l->ff, splits, st, true) : static_cast<int>(BCG_OK);
+  return l->ff > 0 ? project(m, ws->act, l->w_down, ws->proj, ws->proj_floats, T, d, l->ff, splits, st, l) : static_cast<int>(BCG_OK);
 }
 
 // Long launches: queries, keys, values and output gates leave their product as the activations that the matrix memory reads; the
@@ -297,7 +309,7 @@ int stack_step(const bcg_stack* m, const bcg_stack_ws* ws, const bcg_step_batch*
       set_last_error("bcg_stack_step", "unknown mixer");
       return BCG_ERR_UNSUPPORTED;
     }
-    BCG_TRY(project(m, ws->mix, l->w_out, ws->proj, ws->proj_floats, T, d, mix_out, &s, st, true));
+    BCG_TRY(project(m, ws->mix, l->w_out, ws->proj, ws->proj_floats, T, d, mix_out, &s, st, l));
     NormExtra extra;
     extra.bias = l->out_bias;
     const bool has_ff = l->ff > 0 || l->ff_kind == BCG_FF_EXPERTS;
@@ -315,7 +327,7 @@ int stack_step(const bcg_stack* m, const bcg_stack_ws* ws, const bcg_step_batch*
         BCG_TRY(project(m, ws->xn, l->w_up, ws->proj, ws->proj_floats, T, l->ff, d, &s, st));
         BCG_TRY(poly_norm(ws->proj, s, static_cast<long long>(T) * l->ff, l->act_coef, ws->act, dt, T, l->ff, m->eps, st));
       }
-      BCG_TRY(project(m, ws->act, l->w_down, ws->proj, ws->proj_floats, T, d, l->ff, &s, st, true));
+      BCG_TRY(project(m, ws->act, l->w_down, ws->proj, ws->proj_floats, T, d, l->ff, &s, st, l));
       BCG_TRY(sandwich_norm(ws->residual, ws->proj, s, static_cast<long long>(T) * d, l->norm2b, next, ws->xn, dt, T, d,
                             m->eps, {}, st));
     }

@@ -402,3 +402,55 @@ def test_dense_models_step_and_refuse_float32(tmp_path):
     assert (torch.cat(out).cpu() - want).abs().max() < 2e-2
     hf.save_pretrained(str(tmp_path / "hf"), safe_serialization=True)
     assert trace.build_engine(str(tmp_path / "hf"), "float32", 256) is None
+
+
+# One layer each whose output and down products have more than 1,024 inputs, so that launches of more than 128 tokens cut them along K.
+PARTS = {
+    "latent": SM.config([SM.attn(16, 48, 16, 64, 112, 90, ff=2048)], width=1024, vocab=96),
+    "parallel": SM.parallel_config([SM.gattn(8, 2, 64, 64, 90, v_mix=False, mlp=SM.dense(2048))], width=1024, vocab=96),
+    "side": SM.side_config([SM.both(8, 2, 64, 64, mlp=SM.glu(1024), vdim_ssm=128, state=64)], width=1024, vocab=96),
+    "pooled-experts": SM.output_norm_config([SM.pattn(8, 2, 64, 128, 70, 16, 32, mlp=SM.plain_moe(4, 2, 64, 2048))], width=1024, vocab=96),
+}
+
+
+@pytest.mark.parametrize("T", [129, 200, 300])
+@pytest.mark.parametrize("name", PARTS)
+def test_long_launches_with_products_in_parts(name, T):
+    cfg = PARTS[name]
+    m = Model.__new__(Model)
+    m.cfg, m.t, m.dtype = cfg, SM.tensors(cfg, seed=3), "bfloat16"
+    m.eng = SM.engine(cfg, m.t)
+    toks = m.tokens(T)
+    got = m.feed(toks, [T])
+    # the down product came last: its slabs lie in the projections' buffer, and only together they are the product
+    x, w = m.eng.exec, m.eng.w.layers[0]
+    d = 1024
+    out, act = (w["w_down"], x.buf["act"]) if name != "parallel" else (w["w_out"], x.buf["mix"])
+    k = out.shape[1]
+    want = act[:T * k].view(T, k).double() @ out[:d].double().T
+    slabs = x.buf["proj"][:2 * T * d].view(2, T, d).double()
+    near = lambda a: ((a - want).norm() / want.norm()).item()
+    assert near(slabs.sum(0)) < 1e-5 and near(slabs[0]) > 0.1
+    want = m.oracle(toks)
+    m.check(got, want)
+    beside = m.eng.step([(m.eng.open(), toks, list(range(T))), (m.eng.open(), m.tokens(170, 1), [])])     # other parts, by rounding only
+    m.check(beside, want)
+    assert (beside - got).norm() / got.norm() < TOL["bfloat16"] / 2
+
+
+@pytest.mark.parametrize("name", ["latent", "parallel", "pooled-experts"])
+def test_workspace_size_does_not_change_results(name):
+    """The same prompt in engines that differ in how many tokens a launch may have: the same bits.  The feed-forward is small, so that
+    what a workspace of few tokens holds beside a product is less than a second slab."""
+    base = {"latent": SM.config([SM.attn(8, 48, 16, 64, 128, 90, ff=1024)], width=1024, vocab=96),
+            "parallel": SM.parallel_config([SM.gattn(4, 2, 64, 256, 90, v_mix=False, mlp=None)], width=1024, vocab=96),
+            "pooled-experts": SM.output_norm_config([SM.pattn(8, 2, 64, 128, 70, 16, 32, mlp=SM.plain_moe(4, 2, 64, 1024))], width=1024, vocab=96)}
+    cfg, T = base[name], 200
+    t = SM.tensors(cfg, seed=5)
+    toks = torch.randint(0, cfg["vocab"], (T,), generator=torch.Generator().manual_seed(2)).tolist()
+    got = []
+    for tokens in (208, 512, 2048):
+        eng = SM.engine(cfg, t, tokens=256, prefill_tokens=tokens, max_model_len=208)
+        got.append(eng.step([(eng.open(), toks, list(range(T)))]).clone())
+        eng.close()
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
