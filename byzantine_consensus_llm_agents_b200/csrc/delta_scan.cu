@@ -334,7 +334,7 @@ delta_token_kernel(const DeltaArgs a, T* __restrict__ out) {
     }
     // sums of k^2, r.(a*k), r.k; the unit key's factor is applied to the sums
     float part[3] = {kx * kx, r * (rate * kx), r * kx};
-    row_sum<kTokThreads, 1, 3>(sums, part, 0);
+    row_sum<0>(sums, part);
     const float inv = rsqrtf(part[0] + 1e-6f);
     if (i < DP) {
       op[i] = kx;
@@ -360,7 +360,7 @@ delta_token_kernel(const DeltaArgs a, T* __restrict__ out) {
     if (col + oc < D) ss[0] = o * o;
   }
   __syncthreads();                                      // `so`
-  row_sum<kTokThreads, CL, 1>(sh, ss, 0);
+  row_sum<0>(sh, ss);
   const float inv = rsqrtf(ss[0] / static_cast<float>(D) + a.eps);
   for (int i = threadIdx.x; i < kCols; i += kTokThreads) {
     const int ch = cta * kCols + i;

@@ -164,7 +164,7 @@ grouped_norm_in_kernel(const GroupedIn a) {
   if (a.gates)
     for (int h = cta * kInThreads + threadIdx.x; h < a.heads; h += CL * kInThreads)
       a.gates[tok.t * a.heads + h] = a.gate_scale * sigmoid_f32(slab_sum(row + a.gate_col + h, a.n_partials, a.pstride));
-  row_sum<kInThreads, CL, 2>(sh, ss, 0);
+  row_sum<0>(sh, ss);
   const float inv_q = rsqrtf(ss[0] / static_cast<float>(nq) + a.eps);
   const float inv_k = rsqrtf(ss[1] / static_cast<float>(nk - nq) + a.eps);
   for (int c = c0 + threadIdx.x * V; c < c1; c += kInThreads * V) {

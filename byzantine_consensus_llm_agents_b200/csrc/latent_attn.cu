@@ -66,7 +66,7 @@ latent_qkv_kernel(const float* __restrict__ proj, int n_partials, long long pstr
     stage[i] = v;
     ss[0] += v * v;
   }
-  row_sum<kQkvThreads, 1, 1>(sh, ss, 0);
+  row_sum<0>(sh, ss);
   const float inv = rsqrtf(ss[0] / static_cast<float>(kv_rank) + eps);
   T* dst = cache + static_cast<long long>(slot) * (kv_rank + rot_dim);
   for (int i = threadIdx.x; i < kv_rank; i += kQkvThreads) dst[i] = from_f32<T>(stage[i] * inv * latent_norm[i]);
@@ -144,7 +144,7 @@ latent_qkv_vec_kernel(const float* proj, int n_partials, long long pstride, long
     store_vec<4>(stage + i, v);
     ss[0] += v.sumsq();
   }
-  row_sum(sh, ss, 0);
+  row_sum<0>(sh, ss);
   const float inv = rsqrtf(ss[0] / static_cast<float>(kv_rank) + eps);
   for (int i = first; i < kv_rank; i += kQkvThreads * 4) {
     Vec<4> v = load_vec<4>(stage + i);

@@ -102,7 +102,8 @@ __device__ __forceinline__ Vec<V> slab_sum_vec(const float* p, int n, long long 
 }
 
 // Sum of N values over the THREADS x CL threads that share a row (CL CTAs of one cluster); fixed order, so a
-// row's result does not depend on its neighbours.  `slot` must be a fresh 0, 1, ... per call in a kernel.
+// row's result does not depend on its neighbours.  SLOT is another one for each sum of a kernel; in a cluster there are two, each
+// with a barrier for one use.
 //
 // In a cluster every warp sends its sums to every CTA, whose threads wait for the bytes on a barrier of their own: one way
 // through distributed shared memory.  (A barrier of the cluster and eight remote reads behind it took two and the CTA's own barrier.)
@@ -133,8 +134,9 @@ template <int CL>
 __device__ __forceinline__ void row_sum_ready() {
   if constexpr (CL > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
-template <int THREADS, int CL, int N>
-__device__ __forceinline__ void row_sum(RowSum<THREADS, CL, N>& sh, float (&v)[N], int slot, int warps = THREADS / 32) {
+template <int SLOT, int THREADS, int CL, int N>
+__device__ __forceinline__ void row_sum(RowSum<THREADS, CL, N>& sh, float (&v)[N], int warps = THREADS / 32) {
+  static_assert(SLOT >= 0 && (CL == 1 || SLOT < 2), "a third sum would find the first one's barrier complete");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int k = 0; k < N; ++k) v[k] = warp_sum(v[k]);
@@ -150,15 +152,15 @@ __device__ __forceinline__ void row_sum(RowSum<THREADS, CL, N>& sh, float (&v)[N
             "mapa.shared::cluster.u32 dst, %0, %2;\n"
             "mapa.shared::cluster.u32 bar, %1, %2;\n"
             "st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [dst], %3, [bar];\n"
-            "}\n" ::"r"(smem_u32(&sh.warp[slot & 1][k][rank * warps + warp])),
-            "r"(smem_u32(&sh.bar[slot & 1])), "r"(lane), "r"(__float_as_uint(v[k]))
+            "}\n" ::"r"(smem_u32(&sh.warp[SLOT][k][rank * warps + warp])),
+            "r"(smem_u32(&sh.bar[SLOT])), "r"(lane), "r"(__float_as_uint(v[k]))
             : "memory");
     }
-    mbar_wait_cluster(&sh.bar[slot & 1], 0);
+    mbar_wait_cluster(&sh.bar[SLOT], 0);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       float t = 0.f;
-      for (int i = lane; i < CL * warps; i += 32) t += sh.warp[slot & 1][k][i];
+      for (int i = lane; i < CL * warps; i += 32) t += sh.warp[SLOT][k][i];
       v[k] = warp_sum(t);
     }
   } else {

@@ -46,7 +46,7 @@ embed_norm_kernel(const EmbedArgs a, const float* __restrict__ w, float* __restr
     store_vec<V>(residual + t * d + v, x);      // read again below by the same thread
     ss[0] += x.sumsq();
   }
-  row_sum<kRowT, 1, 1>(sh, ss, 0);
+  row_sum<0>(sh, ss);
   float inv = rsqrtf(ss[0] / static_cast<float>(d) + eps);
   if (a.norm) {
     ss[0] = 0.f;
@@ -58,7 +58,7 @@ embed_norm_kernel(const EmbedArgs a, const float* __restrict__ w, float* __restr
       store_vec<V>(residual + t * d + v, x);
       ss[0] += x.sumsq();
     }
-    row_sum<kRowT, 1, 1>(sh, ss, 1);
+    row_sum<1>(sh, ss);
     inv = rsqrtf(ss[0] / static_cast<float>(d) + eps);
   }
   for (int v = threadIdx.x * V; v < d; v += kRowT * V) {
@@ -110,7 +110,7 @@ sandwich_norm_kernel(float* __restrict__ residual, const float* __restrict__ del
   }
   float inv = 1.0f;
   if (w_post) {
-    row_sum<kRowT, CL, 1>(sh, ss, 0);
+    row_sum<0>(sh, ss);
     inv = rsqrtf(ss[0] * inv_d + eps);
   }
   ss[0] = 0.f;
@@ -131,7 +131,7 @@ sandwich_norm_kernel(float* __restrict__ residual, const float* __restrict__ del
     ss[0] += x.sumsq();
   }
   if (w_next) {
-    row_sum<kRowT, CL, 1>(sh, ss, 1);
+    row_sum<1>(sh, ss);
     const float inv2 = rsqrtf(ss[0] * inv_d + eps);
     for (int v = v0 + threadIdx.x * V; v < v1; v += kRowT * V) {
       Vec<V> x = load_vec<V>(stage + v - v0);
@@ -210,7 +210,7 @@ sandwich_row_kernel(float* residual, const float* delta, int n_partials, long lo
   const float inv_d = 1.0f / static_cast<float>(d);
   if (w_post) {
     float ss[1] = {y.sumsq()};
-    row_sum(sh, ss, 0, warps);
+    row_sum<0>(sh, ss, warps);
     const float inv = rsqrtf(ss[0] * inv_d + eps);
 #pragma unroll
     for (int k = 0; k < 4; ++k) x.x[k] = fmaf(y.x[k], inv * wp.x[k], x.x[k]);
@@ -224,7 +224,7 @@ sandwich_row_kernel(float* residual, const float* delta, int n_partials, long lo
   if (mine) store_vec<4>(residual + t * d + 4 * v, x);
   if (w_next) {
     float ss[1] = {x.sumsq()};
-    row_sum(sh, ss, 1, warps);
+    row_sum<1>(sh, ss, warps);
     const float inv = rsqrtf(ss[0] * inv_d + eps);
 #pragma unroll
     for (int k = 0; k < 4; ++k) x.x[k] *= inv * wn.x[k];
@@ -291,7 +291,7 @@ sandwich_long_kernel(float* residual, const float* delta, int n_partials, long l
   if (w_post) {
 #pragma unroll
     for (int j = 0; j < NV; ++j) ss[0] += y[j].sumsq();
-    row_sum(sh, ss, 0);
+    row_sum<0>(sh, ss);
     const float inv = rsqrtf(ss[0] * inv_d + eps);
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
@@ -311,7 +311,7 @@ sandwich_long_kernel(float* residual, const float* delta, int n_partials, long l
     ss[0] = 0.f;
 #pragma unroll
     for (int j = 0; j < NV; ++j) ss[0] += x[j].sumsq();
-    row_sum(sh, ss, 1);
+    row_sum<1>(sh, ss);
     inv = rsqrtf(ss[0] * inv_d + eps);
   }
 #pragma unroll
@@ -338,7 +338,7 @@ rows_norm_kernel(const float* __restrict__ residual, const int* __restrict__ row
   const long long t = blockIdx.x, src = rows[t];
   float ss[1] = {0.f};
   for (int v = threadIdx.x * V; v < d; v += kRowT * V) ss[0] += load_vec<V>(residual + src * d + v).sumsq();
-  row_sum<kRowT, 1, 1>(sh, ss, 0);
+  row_sum<0>(sh, ss);
   const float inv = rsqrtf(ss[0] / static_cast<float>(d) + eps);
   for (int v = threadIdx.x * V; v < d; v += kRowT * V) {
     Vec<V> x = load_vec<V>(residual + src * d + v);
@@ -375,7 +375,7 @@ poly_norm_kernel(const float* __restrict__ z, int n_partials, long long partial_
       s[2] = fmaf(x4, x2, s[2]);
     }
   }
-  row_sum<kRowT, CL, 3>(sh, s, 0);
+  row_sum<0>(sh, s);
   const float inv_f = 1.0f / static_cast<float>(ff);
   const float a = coef[0] * rsqrtf(s[0] * inv_f + eps), b = coef[1] * rsqrtf(s[1] * inv_f + eps),
               c = coef[2] * rsqrtf(s[2] * inv_f + eps), e = coef[3];
@@ -421,7 +421,7 @@ poly_row_kernel(const float* z, int n_partials, long long partial_stride, const 
       s[2] = fmaf(x4, x2, s[2]);
     }
   row_sum_ready<CL>();
-  row_sum(sh, s, 0);
+  row_sum<0>(sh, s);
   const float inv_f = 1.0f / static_cast<float>(ff);
   const float a = c0 * rsqrtf(s[0] * inv_f + eps), b = c1 * rsqrtf(s[1] * inv_f + eps), c = c2 * rsqrtf(s[2] * inv_f + eps);
 #pragma unroll

@@ -648,7 +648,7 @@ ssm_norm_kernel(const SsmArgs a, T* __restrict__ out, long long out_ld) {
     store_vec<V>(stage + v - v0, u);
     ss[0] += u.sumsq();
   }
-  row_sum(sh, ss, 0);
+  row_sum<0>(sh, ss);
   const float inv = rsqrtf(ss[0] / static_cast<float>(width) + a.eps);
   for (int v = first; v < v1; v += kSnThreads * V) {
     Vec<V> x = load_vec<V>(stage + v - v0);

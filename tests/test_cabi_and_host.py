@@ -253,3 +253,30 @@ def test_sums_from_other_ctas_are_waited_for_at_cluster_scope():
     assert found
     wait = re.search(r"bool mbar_try_wait_cluster\(.*?\n}\n", (ROOT / "byzantine_consensus_llm_agents_b200/csrc/common.cuh").read_text(), re.S)
     assert "acquire.cluster" in wait.group(0)
+
+
+@pytest.mark.parametrize("slot,compiles", [(1, True), (2, False)])
+def test_a_cluster_sums_at_most_twice_per_kernel(slot, compiles, tmp_path):
+    """Each of a cluster's two barriers completes once: a third sum would read what has not arrived.  The compiler says so."""
+    import subprocess
+
+    from byzantine_consensus_llm_agents_b200 import build as B
+    try:
+        nvcc = B._nvcc()
+    except RuntimeError:
+        pytest.skip("no nvcc")
+    src = tmp_path / "sums.cu"
+    src.write_text(f"""#include "stack_common.cuh"
+__global__ void sums(float* x) {{
+  __shared__ bcg::RowSum<128, 8, 1> sh;
+  float v[1] = {{x[threadIdx.x]}};
+  bcg::row_sum_begin(sh);
+  bcg::row_sum_ready<8>();
+  bcg::row_sum<{slot}>(sh, v);
+  x[threadIdx.x] = v[0];
+}}
+""")
+    r = subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "--expt-relaxed-constexpr", "-O0", f"-I{B.CSRC}",
+                        f"-I{ROOT / 'include'}", "-c", str(src), "-o", str(tmp_path / "sums.o")], capture_output=True, text=True)
+    assert (r.returncode == 0) == compiles, r.stderr[-2000:]
+    assert compiles or "third sum" in r.stderr
