@@ -417,11 +417,11 @@ class Engine:
                 if self.enable_prefix_cache:
                     hs = PagePool.chains(ids)
                     pages = self.pool.acquire_prefix(hs[:(len(ids) - 1) // PAGE])   # always compute at least the last prompt token
+                pages_of.append(pages)      # before it grows: what is held is given back if the pool runs out
                 hit = len(pages)
                 total_pages = (len(ids) + q.max_tokens + PAGE - 1) // PAGE
                 while len(pages) < total_pages:
                     pages.append(self.pool.alloc())
-                pages_of.append(pages)
                 blocks_of.append([[] for _ in self.block_pools])
                 self._grow_blocks(blocks_of[-1], len(ids) + q.max_tokens)
                 hashes_of.append(hs)

@@ -280,3 +280,30 @@ __global__ void sums(float* x) {{
                         f"-I{ROOT / 'include'}", "-c", str(src), "-o", str(tmp_path / "sums.o")], capture_output=True, text=True)
     assert (r.returncode == 0) == compiles, r.stderr[-2000:]
     assert compiles or "third sum" in r.stderr
+
+
+def _wave_engine(pages, prefix_cache=True):
+    """An engine's host side, as far as a wave's page layout goes."""
+    from types import SimpleNamespace
+
+    from byzantine_consensus_llm_agents_b200.engine import Engine, PagePool, SlotPool
+    e = Engine.__new__(Engine)
+    e.cfg, e.row, e.max_model_len, e.enable_prefix_cache = None, {}, 4096, prefix_cache
+    e.exec, e.pool, e.block_pools, e.slots = SimpleNamespace(block_pools=[], has_state=False), PagePool(pages), [], SlotPool(4)
+    return e
+
+
+def test_pages_are_given_back_when_the_pool_runs_out(so):
+    """The pool ends in the middle of a wave's second request, behind pages of its cached prefix: all references are given back."""
+    from byzantine_consensus_llm_agents_b200.engine import PAGE, PagePool, Request
+    e = _wave_engine(12)
+    prompt = list(range(5 * PAGE + 3))
+    for h in PagePool.chains(prompt)[:3]:
+        p = e.pool.alloc()
+        e.pool.publish(p, h)
+        e.pool.release(p)
+    small, large = Request("", prompt_ids=[9] * 20, max_tokens=8), Request("", prompt_ids=prompt, max_tokens=20 * PAGE)
+    for _ in range(2):
+        with pytest.raises(MemoryError):
+            e._generate_wave([small, large], 0)
+        assert not e.pool.ref and len(e.pool.free) + len(e.pool.cached) == 12
