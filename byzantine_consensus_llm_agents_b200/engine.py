@@ -95,13 +95,19 @@ class PagePool:
         return hashlib.blake2b(prev + struct.pack(f"<{len(block)}i", *block), digest_size=16).digest()
 
     @staticmethod
+    def packed(ids: Sequence[int]) -> bytes:
+        """The tokens of a prompt's full blocks; what is not a 32-bit whole number is refused (struct.error)."""
+        n = len(ids) // PAGE * PAGE
+        return struct.pack(f"<{n}i", *ids[:n])
+
+    @staticmethod
     def chains(ids: Sequence[int]) -> Sequence[bytes]:
         """chain() over all full blocks of a prompt, in one native call."""
         n = len(ids) // PAGE
         if not n:
             return ()
         out = C.create_string_buffer(16 * n)
-        L.check(L.load().bcg_block_hashes(struct.pack(f"<{n * PAGE}i", *ids[:n * PAGE]), n, PAGE, out), "bcg_block_hashes")
+        L.check(L.load().bcg_block_hashes(PagePool.packed(ids), n, PAGE, out), "bcg_block_hashes")
         return struct.unpack("16s" * n, out.raw)
 
     def acquire_prefix(self, hashes: Sequence[bytes]) -> List[int]:
@@ -417,6 +423,8 @@ class Engine:
                 if self.enable_prefix_cache:
                     hs = PagePool.chains(ids)
                     pages = self.pool.acquire_prefix(hs[:(len(ids) - 1) // PAGE])   # always compute at least the last prompt token
+                else:
+                    PagePool.packed(ids)        # the device's tokens are 32-bit numbers, hashed or not
                 pages_of.append(pages)      # before it grows: what is held is given back if the pool runs out
                 hit = len(pages)
                 total_pages = (len(ids) + q.max_tokens + PAGE - 1) // PAGE

@@ -307,3 +307,16 @@ def test_pages_are_given_back_when_the_pool_runs_out(so):
         with pytest.raises(MemoryError):
             e._generate_wave([small, large], 0)
         assert not e.pool.ref and len(e.pool.free) + len(e.pool.cached) == 12
+
+
+@pytest.mark.parametrize("prefix_cache", [True, False])
+@pytest.mark.parametrize("bad", [2 ** 31, -2 ** 31 - 1, 1.5])
+def test_tokens_that_are_not_32_bit_numbers_are_refused(so, prefix_cache, bad):
+    """With or without a prefix cache: they would wrap on their way to the device."""
+    import struct
+
+    from byzantine_consensus_llm_agents_b200.engine import Request
+    e = _wave_engine(12, prefix_cache)
+    with pytest.raises(struct.error):
+        e._generate_wave([Request("", prompt_ids=[1] * 7 + [bad] + [2] * 20, max_tokens=4)], 0)
+    assert not e.pool.ref
