@@ -775,8 +775,9 @@ int state_space(const bcg_stack* m, const bcg_layer* l, const bcg_stack_ws* ws, 
   if (!l->conv_w || !l->conv_b || !l->step_bias || !l->decay_rate || !l->skip || !l->ssm_norm || !l->ssm_state ||
       (l->ssm_taps > 1 && !l->conv_state) || !ws->ssm_x || !ws->ssm_step || !ws->ssm_y || !b->state_slots || l->ssm_n <= 0 ||
       l->ssm_n > 256 || l->ssm_vdim <= 0 || l->ssm_taps < 1 || l->ssm_groups <= 0 || l->ssm_heads % l->ssm_groups ||
-      l->ssm_norm_parts <= 0 || (l->ssm_heads * l->ssm_vdim) % l->ssm_norm_parts || l->ssm_heads * l->ssm_vdim / l->ssm_norm_parts > 51200 || b->n_seqs > 65535) {
-    set_last_error("bcg_state_space", "bad layer (1..256 state entries, groups and parts that divide) or too many sequences");
+      l->ssm_norm_parts <= 0 || (l->ssm_heads * l->ssm_vdim) % l->ssm_norm_parts || l->ssm_heads * l->ssm_vdim / l->ssm_norm_parts > 51200 ||
+      b->n_seqs <= 0 || b->n_seqs > 65535) {
+    set_last_error("bcg_state_space", "bad layer (1..256 state entries, groups and parts that divide), no sequences or too many");
     return BCG_ERR_ARG;
   }
   SsmArgs a = {};

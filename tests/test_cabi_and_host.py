@@ -320,3 +320,18 @@ def test_tokens_that_are_not_32_bit_numbers_are_refused(so, prefix_cache, bad):
     with pytest.raises(struct.error):
         e._generate_wave([Request("", prompt_ids=[1] * 7 + [bad] + [2] * 20, max_tokens=4)], 0)
     assert not e.pool.ref
+
+
+def test_state_space_without_sequences_is_refused_before_any_launch(so):
+    """Tokens of no sequence: the chunks' form divides by the count of sequences on the host."""
+    layer, m, ws, b = L.Layer(), L.Stack(), L.StackWs(), L.StepBatch()
+    for s in (layer, m, ws, b):                  # pointers that nobody follows, sizes that fit
+        for name, kind in s._fields_:
+            if kind is C.c_void_p:
+                setattr(s, name, 16)
+    m.n_layers, m.d_model, m.page_size, m.act_dtype, m.layers = 1, 64, 16, L.DT_BF16, C.pointer(layer)
+    layer.mixer, layer.ssm_heads, layer.ssm_vdim, layer.ssm_n, layer.ssm_groups, layer.ssm_taps, layer.ssm_norm_parts = \
+        L.MIXER_STATE_SPACE, 1, 64, 64, 1, 4, 1
+    b.T, b.n_seqs, ws.T_max = 600, 0, 1024
+    assert so.bcg_state_space(C.byref(m), C.byref(ws), C.byref(b), 0, 1, 0, 64, 0, None) == 1        # a bad argument
+    assert b"no sequences" in so.bcg_last_error()
