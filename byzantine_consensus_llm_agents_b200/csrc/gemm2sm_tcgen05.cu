@@ -397,8 +397,7 @@ int gemm_long_splits(int M, int N, int K, long long room) {
 }
 
 // Returns BCG_ERR_UNSUPPORTED when the shape is not for this kernel (the caller then uses the
-// single-CTA kernel).  From 129 rows on: up to 511 the single-CTA kernel's 128 x 256 tiles ran before, which read 48 KB per
-// k-block and SM where a pair's CTA reads 32 KB for as much work.
+// single-CTA kernel).
 int gemm2sm_bf16_tn(const void* X, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,
                     long long ld_out, int epi, int splits, float glu_limit, float glu_alpha, cudaStream_t stream) {
   if (!for_pairs(M, N) || (splits > 1 && epi != BCG_EPI_F32)) return BCG_ERR_UNSUPPORTED;

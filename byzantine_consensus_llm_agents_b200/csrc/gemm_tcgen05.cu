@@ -653,6 +653,21 @@ int gemm_splits_for(int M, int N, int K) {
 
 // Tiles of 256 columns where they cover no more than tiles of 128 would.
 static bool wide_tiles(int N) { return (N + 255) / 256 * 2 == (N + 127) / 128; }
+// Columns of a long launch's tiles on single SMs
+static int long_columns(int N, int epi) { return wide_tiles(N) && !(epi == BCG_EPI_F32 && N < 2048) ? 256 : 128; }
+
+// Pairs of SMs (256 x 256 tiles) or single ones (128 x 256, or 128 x 128) for launches of 129 to 511 rows.  A pair's k-block is cheaper
+// (its CTAs read 32 KB for what costs a single one 48), its start and end dearer, and its tail of a round larger.  In microseconds,
+// from 23 products of the presets' and stacks' widths at 129 to 511 rows: 13 + 0.30 per k-block and round, 11 + 0.38, or 0.26 for tiles
+// of 128 columns.  Pairs / singles: 256 x 4096 -> 4096 32.8 / 36.9, 300 x 4096 -> 24576 84.0 / 81.9, 300 x 2048 -> 10304 34.8 / 27.6,
+// 256 x 2048 -> 1024 23.6 / 16.4, 448 x 4096 -> 24576 86 / 102.
+static bool pairs_are_faster(int M, int N, int K, int epi) {
+  const int bn = long_columns(N, epi), kb = (K + kBlockK - 1) / kBlockK, sms = num_sms();
+  const int singles = ((M + 127) / 128) * ((N + bn - 1) / bn), pairs = ((M + 255) / 256) * ((N + 255) / 256);
+  const double one = 11.0 + (singles + sms - 1) / sms * kb * (bn == 256 ? 0.38 : 0.26);
+  const double two = 13.0 + (pairs + sms / 2 - 1) / (sms / 2) * kb * 0.30;
+  return two < one;
+}
 
 static int gemm_dense(const void* X, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,
                       long long ld_out, int epi, int splits, int flags, const bcg_gemm_fusion* fu, float glu_limit,
@@ -714,7 +729,7 @@ static int gemm_dense(const void* X, const void* W, void* out, int M, int N, int
     set_last_error("bcg_gemm_bf16_tn", "ld_out must keep 16-byte row alignment");
     return BCG_ERR_ARG;
   }
-  if (!swap && !(fu && (fu->scale_sumsq || fu->red_counters))) {
+  if (!swap && !(fu && (fu->scale_sumsq || fu->red_counters)) && (M >= 512 || splits > 1 || pairs_are_faster(M, N, K, epi))) {
     // prefill-sized: 256x256 tiles on CTA pairs when the shape allows it
     const int rc2 = gemm2sm_bf16_tn(X, W, out, M, N, K, ldx, ldw, ld_out, epi, splits, glu_limit, glu_alpha, stream);
     if (rc2 != BCG_ERR_UNSUPPORTED) return rc2;
@@ -774,8 +789,7 @@ static int gemm_dense(const void* X, const void* W, void* out, int M, int N, int
     a.hint_a = kEvictFirst;  // weights are streamed exactly once per step
     a.hint_b = kEvictLast;
   } else {
-    bn = wide_tiles(N) ? 256 : 128;
-    if (epi == BCG_EPI_F32 && bn == 256 && N < 2048) bn = 128;
+    bn = long_columns(N, epi);
     a.tiles_a = (M + kBlockA - 1) / kBlockA;
     a.tiles_b = (N + bn - 1) / bn;
     a.group_a = 16;

@@ -138,6 +138,24 @@ def test_gemm_batch_invariance():
         assert torch.equal(outs[0], o)
 
 
+@pytest.mark.parametrize("epi", ["EPI_F32", "EPI_BF16", "EPI_SWIGLU"])
+@pytest.mark.parametrize("N,K", [(1024, 200), (2048, 64), (4128, 520), (10304, 264)])
+def test_gemm_long_launches_on_pairs_and_single_sms(N, K, epi):
+    """Launches of 129 to 511 rows run on pairs of SMs or on single ones, whichever the shape suits, those of 512 on pairs: a row's
+    result is the same bits either way."""
+    code = getattr(L, epi)
+    x, w = _rand_bf16(512, K, seed=41), _rand_bf16(N, K, scale=0.05, seed=42)
+    new = lambda M: torch.full((M, N // 2 if epi == "EPI_SWIGLU" else N), float("nan"), device=DEV,
+                               dtype=torch.float32 if epi == "EPI_F32" else torch.bfloat16)
+    want = new(512)
+    L.gemm(x, w, want, code)
+    assert torch.isfinite(want.float()).all()
+    for M in (129, 256, 257, 300, 384, 385, 511):
+        out = new(M)
+        L.gemm(x[:M], w, out, code)
+        assert torch.equal(out, want[:M]), M
+
+
 def test_gemm_rejects_bad_args():
     x = _rand_bf16(4, 64)
     w = _rand_bf16(128, 64)
