@@ -275,13 +275,15 @@ add_norm_stats_kernel(float* __restrict__ residual, const void* __restrict__ del
   }
 }
 
-// One 128-thread CTA per row (16 of them fit on an SM: the launch is bandwidth-bound, where the
-// earlier 1024-thread version reached a third of the HBM rate).  Physical warp pw plays the
-// virtual warps pw, pw + 4, ... of the order described above; the summed row is staged in shared
-// memory between the statistics pass and the scaling pass.
+// One 128-thread CTA per row.  Physical warp pw plays the virtual warps pw, pw + 4, ... of the order described above; the summed row
+// is staged in shared memory between the statistics pass and the scaling pass.
+// AHEAD: one fp32 slab and one turn (prompts of all models here); the next virtual warp's vector is read while this one's is summed, so
+// that a thread has two in flight, in ten CTAs per SM (without it a 5120-wide row had too few reads under way): 12,390 rows of 5120
+// 211 -> 176 us.  The other forms want more registers than ten CTAs leave (bf16 rows of 8192: 293 us, squeezed 324).
 constexpr int kRowThreads = 128;
 
-__global__ void __launch_bounds__(kRowThreads, 10)
+template <bool AHEAD>
+__global__ void __launch_bounds__(kRowThreads, AHEAD ? 10 : 0)
 add_rmsnorm_row_kernel(float* __restrict__ residual, const void* __restrict__ delta, int delta_is_f32,
                        int n_partials, long long partial_stride, const float* __restrict__ w,
                        __nv_bfloat16* __restrict__ xn, const int* __restrict__ src_rows, int d,
@@ -297,22 +299,19 @@ add_rmsnorm_row_kernel(float* __restrict__ residual, const void* __restrict__ de
   const int nvec = d >> 2;
   const int per = (nvec + kNormSegments - 1) / kNormSegments;
   const int pw = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // One fp32 slab and one turn (prompts of all models here): the next virtual warp's vector is read while this one's is summed, so
-  // that a thread has two in flight (11 CTAs of a 5120-wide row per SM had too few).  12,390 rows of 5120: 252 -> 181 us.
-  const bool ahead = delta && delta_is_f32 && n_partials == 1 && per <= kSegThreads;
-  float4 rn = make_float4(0.f, 0.f, 0.f, 0.f), pn = rn;
-  auto vector_of = [&](int vw) {      // -1: none
-    const int vt = (vw & 7) * 32 + lane, v = (vw >> 3) * per + vt;
-    return vw < kVirtWarps && vt < per && v < nvec ? v : -1;
-  };
-  auto fetch = [&](int vw) {
-    const int v = vector_of(vw);
-    if (v >= 0) {
-      rn = *reinterpret_cast<const float4*>(residual + src * d + v * 4);
-      pn = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(delta) + src * d + v * 4);
-    }
-  };
-  if (ahead) {
+  if constexpr (AHEAD) {
+    float4 rn = make_float4(0.f, 0.f, 0.f, 0.f), pn = rn;
+    auto vector_of = [&](int vw) {      // -1: none
+      const int vt = (vw & 7) * 32 + lane, v = (vw >> 3) * per + vt;
+      return vw < kVirtWarps && vt < per && v < nvec ? v : -1;
+    };
+    auto fetch = [&](int vw) {
+      const int v = vector_of(vw);
+      if (v >= 0) {
+        rn = *reinterpret_cast<const float4*>(residual + src * d + v * 4);
+        pn = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(delta) + src * d + v * 4);
+      }
+    };
     fetch(pw);
     for (int vw = pw; vw < kVirtWarps; vw += kPhysWarps) {
       const float4 x = make_float4(rn.x + pn.x, rn.y + pn.y, rn.z + pn.z, rn.w + pn.w);
@@ -328,26 +327,27 @@ add_rmsnorm_row_kernel(float* __restrict__ residual, const void* __restrict__ de
       }
       if (lane == 0) red[vw] = ss;
     }
-  }
-  for (int vw = ahead ? kVirtWarps : pw; vw < kVirtWarps; vw += kPhysWarps) {
-    const int seg = vw >> 3;
-    const int vt = (vw & 7) * 32 + lane;
-    float ss = 0.f;
-    if ((vw & 7) * 32 < per) {  // virtual warps past the segment's end contribute exact zeros
-      const int v_end = min(nvec, (seg + 1) * per);
+  } else {
+    for (int vw = pw; vw < kVirtWarps; vw += kPhysWarps) {
+      const int seg = vw >> 3;
+      const int vt = (vw & 7) * 32 + lane;
+      float ss = 0.f;
+      if ((vw & 7) * 32 < per) {  // virtual warps past the segment's end contribute exact zeros
+        const int v_end = min(nvec, (seg + 1) * per);
 #pragma unroll
-      for (int i = 0; i < kSegTurns; ++i) {
-        const int v = seg * per + vt + i * kSegThreads;
-        if (vt + i * kSegThreads < per && v < v_end) {
-          const float4 x = residual_plus_delta<4>(residual, delta, delta_is_f32, n_partials,
-                                                  partial_stride, src * d + v * 4);
-          row_stage[v] = x;
-          ss = __fadd_rn(ss, sumsq4(x));
+        for (int i = 0; i < kSegTurns; ++i) {
+          const int v = seg * per + vt + i * kSegThreads;
+          if (vt + i * kSegThreads < per && v < v_end) {
+            const float4 x = residual_plus_delta<4>(residual, delta, delta_is_f32, n_partials,
+                                                    partial_stride, src * d + v * 4);
+            row_stage[v] = x;
+            ss = __fadd_rn(ss, sumsq4(x));
+          }
         }
+        ss = warp_sum(ss);
       }
-      ss = warp_sum(ss);
+      if (lane == 0) red[vw] = ss;
     }
-    if (lane == 0) red[vw] = ss;
   }
   __syncthreads();
   float tot = 0.f;
@@ -623,10 +623,11 @@ int add_rmsnorm(float* residual, const void* delta, int delta_is_f32, int n_part
                             stream, residual, delta, delta_is_f32, n_partials, partial_stride, w,
                             reinterpret_cast<__nv_bfloat16*>(xn), src_rows, d, eps));
   } else {
-    if (const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(add_rmsnorm_row_kernel),
-                                           kNormSegments * kSegThreads * kSegTurns * 16))
+    const bool ahead = delta && delta_is_f32 && n_partials == 1 && d <= kNormSegments * kSegThreads * 4;     // one turn
+    const auto kernel = ahead ? add_rmsnorm_row_kernel<true> : add_rmsnorm_row_kernel<false>;
+    if (const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kNormSegments * kSegThreads * kSegTurns * 16))
       return rc;
-    BCG_CUDA_CHECK(launch_k(add_rmsnorm_row_kernel, dim3(T), dim3(kRowThreads), static_cast<size_t>(d) * 4,
+    BCG_CUDA_CHECK(launch_k(kernel, dim3(T), dim3(kRowThreads), static_cast<size_t>(d) * 4,
                             stream, residual, delta, delta_is_f32, n_partials, partial_stride, w,
                             reinterpret_cast<__nv_bfloat16*>(xn), src_rows, d, eps));
   }

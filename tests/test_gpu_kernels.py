@@ -351,6 +351,12 @@ def test_add_rmsnorm_row_is_independent_of_launch_size(d, parts):
     assert torch.equal(xn_m[pick].view(torch.int16), xn_f.view(torch.int16))
 
 
+@pytest.mark.parametrize("d", [4, 1000, 5120, 8192, 8196, 16384])
+def test_add_rmsnorm_row_of_one_slab_is_independent_of_launch_size(d):
+    """One fp32 slab, the form of prompts: read a vector ahead up to 8,192 columns, in turns beyond."""
+    test_add_rmsnorm_row_is_independent_of_launch_size(d, 1)
+
+
 @pytest.mark.parametrize("T,d,parts", [(10, 5120, 11), (1, 256, 1), (128, 1024, 3), (7, 6144, 0), (5, 1000, 2)])
 def test_add_norm_stats_plus_consumer_scale_equals_add_rmsnorm(T, d, parts):
     """bcg_add_norm_stats leaves the residual exactly as bcg_add_rmsnorm does, xn = bf16(r*w), and
