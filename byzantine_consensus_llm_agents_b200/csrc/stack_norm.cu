@@ -487,8 +487,10 @@ static int sandwich_t(float* residual, const float* delta, int n_partials, long 
   } else if (cl) {
     BCG_CUDA_CHECK(launch_cluster(sandwich_norm_kernel<T, V, kRowCluster>, dim3(kRowCluster, T_rows), dim3(kRowT),
                                   kRowCluster, sm, st, residual, delta, n_partials, stride, w_post, w_next, x, d, eps, extra));
-  } else if (V == 4 && T_rows > kClusterMaxRows && d <= 8192) {
-    const auto kernel = d <= 2048 ? sandwich_long_kernel<T, 128, 4> : d <= 4096 ? sandwich_long_kernel<T, 256, 4> : sandwich_long_kernel<T, 256, 8>;
+  } else if (V == 4 && T_rows > kClusterMaxRows && d <= 4096) {
+    // wider rows take eight vectors per thread, and staging them is faster: 2,000 rows of 5120 38.9 us staged, 41.0 in registers,
+    // 6,000 of 8192 149.5 and 161.8
+    const auto kernel = d <= 2048 ? sandwich_long_kernel<T, 128, 4> : sandwich_long_kernel<T, 256, 4>;
     BCG_CUDA_CHECK(launch_k(kernel, dim3(T_rows), dim3(d <= 2048 ? 128 : 256), 0, st, residual, delta, n_partials, stride, w_post, w_next, x,
                             d, eps, extra));
   } else {

@@ -388,11 +388,18 @@ def test_gemm_any_infinite_weights(M, N, K):
     torch.testing.assert_close(got[ok], want[ok], rtol=1e-5, atol=1e-4)
 
 
-# Long launches keep a row in registers: the widest row of each form, ragged ends, several slabs, and the next width.
+# Long launches keep a row in registers, wide ones in shared memory: the widest row of each form, ragged ends, several slabs, and the
+# next width.
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("T,d,parts", [(129, 2048, 3), (140, 2052, 1), (129, 4096, 2), (131, 8192, 1), (129, 8196, 2), (150, 4, 1)])
 def test_sandwich_norm_of_long_launches(dtype, T, d, parts):
     test_sandwich_norm(dtype, T, d, parts)
+
+
+@pytest.mark.parametrize("T,d,parts", [(130, 4100, 3), (300, 5120, 1)])
+def test_sandwich_norm_of_wide_long_launches(T, d, parts):
+    for dtype in DT:
+        test_sandwich_norm(dtype, T, d, parts)
 
 
 @pytest.mark.parametrize("dtype", DT)
