@@ -588,7 +588,7 @@ int make_tmap_bf16_sw128(CUtensorMap* m, const void* ptr, long long rows, long l
   return BCG_OK;
 }
 
-static int num_sms() {
+int num_sms() {
   static int n = 0;
   if (n == 0) {
     int dev = 0;

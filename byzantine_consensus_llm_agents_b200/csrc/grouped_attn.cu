@@ -935,14 +935,24 @@ static GroupedAttn attn_args(const bcg_stack* m, const bcg_layer* l, const bcg_s
   return a;
 }
 
+// Tiles of 32 tokens or a CTA per token and head?  A tile walks the contexts of its sequences one behind another, where a token's CTA
+// has its own; over the same context a tile takes 2.9 times as long as a token's CTA.  Both have two CTAs per SM.  16 heads of 128,
+// contexts of 1,500, tiles / tokens: 1 x 64 tokens 213 / 333 us, 1 x 32 211 / 147, 8 x 16 327 / 662, 8 x 8 630 / 341, 8 x 3 1224 / 130.
+static bool tiles_are_faster(int n, int n_seqs, int heads) {
+  if (n_seqs <= 0 || n <= n_seqs) return false;
+  const long long slots = 2 * num_sms(), tiles = (n + kGtQueries - 1) / kGtQueries, tokens = n < kGtQueries ? n : kGtQueries;
+  const long long walked = (tokens * n_seqs + n - 1) / n;       // sequences of a tile, on average
+  return 2.9 * static_cast<double>(walked * ((tiles * heads + slots - 1) / slots)) <=
+         static_cast<double>((static_cast<long long>(n) * heads + slots - 1) / slots);
+}
+
 static int grouped_plain(const bcg_stack* m, const bcg_layer* l, const bcg_stack_ws* ws, const bcg_step_batch* b,
                          const int* rows, int n, cudaStream_t st) {
   const GroupedAttn a = attn_args(m, l, ws, b, rows);
-  // Prompts' tokens share keys; among tokens that each have a sequence of their own there is nothing to share.
-  if (m->act_dtype == BCG_DT_F32 && !rows && b->row_seq && n >= 2 * b->n_seqs && l->pool == 0 && !a.v_cos_sin && l->dim % 4 == 0 &&
+  if (m->act_dtype == BCG_DT_F32 && !rows && b->row_seq && l->pool == 0 && !a.v_cos_sin && l->dim % 4 == 0 &&
       l->vdim % 4 == 0 && l->dim <= kGtDim && l->vdim <= kGtDim && l->q_ld % 4 == 0 && l->v_ld % 4 == 0 && l->mix_ld % 4 == 0 &&
       ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache) |
-        reinterpret_cast<uintptr_t>(a.out)) & 15) == 0) {
+        reinterpret_cast<uintptr_t>(a.out)) & 15) == 0 && tiles_are_faster(n, b->n_seqs, l->heads)) {
     BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_tile_kernel), kGtSmem));
     BCG_CUDA_CHECK(launch_k(grouped_tile_kernel, dim3((n + kGtQueries - 1) / kGtQueries, l->heads), dim3(kGtThreads), kGtSmem, st, a, n));
     return BCG_OK;

@@ -41,6 +41,7 @@ int gemm_any_grouped(const void* X, int x_dtype, const void* W, float* out, int 
 int gemm2sm_bf16_tn(const void* X, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,
                     long long ld_out, int epi, int splits, float glu_limit, float glu_alpha, cudaStream_t stream);
 int gemm_long_splits(int M, int N, int K, long long room);
+int num_sms();      // of the device (148 where there is none)
 // TMA descriptor of a row-major bf16 matrix (rows x K, pitch ld elements): boxes of box_rows x 64
 // elements land in shared memory 128B-swizzled, out-of-bounds elements read as zero.
 int make_tmap_bf16_sw128(CUtensorMap* m, const void* ptr, long long rows, long long K, long long ld,

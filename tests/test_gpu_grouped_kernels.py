@@ -156,13 +156,21 @@ def test_grouped_attention_fp32_tiles(size, window):
     _check(a, _seqs(a, ((130, 33), (65, 64), (64, 1), (40, 3), (31, 31)), window), 3e-6)
 
 
+@pytest.mark.parametrize("size", ["small", "usual", "max"])
+@pytest.mark.parametrize("window", [0, 1, 33, 65])
+def test_grouped_attention_fp32_of_many_tokens(size, window):
+    """Tokens enough for tiles to be the faster form, among them parts of sequences that are shorter than a tile."""
+    a = Attention(size, window, "float32", tokens=1024, rows=8)
+    _check(a, _seqs(a, ((300, 200), (40, 21), (64, 1), (9, 3), (150, 150), (65, 64), (73, 73)), window), 3e-6)
+
+
 @pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
 @pytest.mark.parametrize("window", [0, 17])
 def test_values_that_are_not_finite_reach_only_the_tokens_that_see_them(value, window):
     """Two tokens of the second sequence have a value that is infinite or NaN; the first and third sequence share CTAs, and warps of
     four queries, with it.  Whoever does not see them is exact as ever, and so are all other columns."""
-    a = Attention("usual", window, "float32")
-    seqs = _seqs(a, ((40, 21), (70, 34), (43, 43)), window)
+    a = Attention("usual", window, "float32", tokens=1024)
+    seqs = _seqs(a, ((40, 21), (70, 34), (43, 43), (400, 400)), window)      # tokens enough for tiles
     odd = (45, 60)
     for j in odd:
         seqs[1][1][j, :, 3] = value
