@@ -602,7 +602,7 @@ int grouped_in(const bcg_stack* m, const bcg_layer* l, const bcg_stack_ws* ws, c
 }
 
 // ------------------------------------------------------------------------------------------- plain
-constexpr int kGpThreads = 512, kGpKeys = 256, kGpWarps = kGpThreads / 32, kGpAhead = 4;
+constexpr int kGpThreads = 512, kGpShort = 128, kGpKeys = 256, kGpAhead = 4;
 
 struct GroupedAttn {
   const void *q, *k_cache, *v_cache;
@@ -634,9 +634,11 @@ __host__ __device__ __forceinline__ int plain_groups(int dim, int vdim) {
 
 // Keys' rows are looked up once per chunk, a warp has kGpAhead keys' reads in flight, and the values' columns are read by as many
 // groups of threads as the CTA has, a part of the keys each.  Single tokens at 410 keys, 16 heads: 80 -> 30 us.
-template <typename T>
-__global__ void __launch_bounds__(kGpThreads)
+// THREADS: kGpShort for up to 32 keys, which one warp's weights cover; groups then take turns, so that every sum keeps its order.
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 grouped_plain_kernel(const GroupedAttn a) {
+  constexpr int kGpWarps = THREADS / 32;
   extern __shared__ float sm[];
   __shared__ float red[kGpWarps];
   __shared__ long long key_row[kGpKeys];
@@ -654,8 +656,8 @@ grouped_plain_kernel(const GroupedAttn a) {
   const float slope = a.slopes ? a.slopes[h] : 0.f;
   const int groups = plain_groups(a.dim, a.vdim), width = groups > 1 ? kGpThreads / groups : kGpThreads;
   const int group = threadIdx.x / width, column = threadIdx.x % width;
-  for (int i = threadIdx.x; i < a.dim; i += kGpThreads) qs[i] = to_f32<T>(qh[i]);
-  for (int i = threadIdx.x; i < groups * a.vdim; i += kGpThreads) oc[i] = 0.f;
+  for (int i = threadIdx.x; i < a.dim; i += THREADS) qs[i] = to_f32<T>(qh[i]);
+  for (int i = threadIdx.x; i < groups * a.vdim; i += THREADS) oc[i] = 0.f;
   float m = -INFINITY, l = 0.f;
   const int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
   // tokens lo .. pos, then the pooled blocks that are seen
@@ -666,7 +668,7 @@ grouped_plain_kernel(const GroupedAttn a) {
   for (int j0 = 0; j0 < n_all; j0 += kGpKeys) {
     const int n = min(kGpKeys, n_all - j0);
     __syncthreads();
-    for (int j = threadIdx.x; j < n; j += kGpThreads) key_row[j] = row_of(j0 + j);
+    for (int j = threadIdx.x; j < n; j += THREADS) key_row[j] = row_of(j0 + j);
     __syncthreads();
     float mx = -INFINITY;
     for (int j = warp * kGpAhead; j < n; j += kGpWarps * kGpAhead) {
@@ -693,7 +695,7 @@ grouped_plain_kernel(const GroupedAttn a) {
     const float m_new = fmaxf(m, mx);
     const float corr = expf(m - m_new);
     float sum = 0.f;
-    for (int j = threadIdx.x; j < n; j += kGpThreads) {
+    for (int j = threadIdx.x; j < n; j += THREADS) {
       const float e = expf(p[j] - m_new);
       p[j] = e;
       sum += e;
@@ -707,14 +709,25 @@ grouped_plain_kernel(const GroupedAttn a) {
     for (int i = 0; i < kGpWarps; ++i) sum += red[i];
     l = l * corr + sum;
     m = m_new;
-    if (group < groups)
-      for (int r = column; r < a.vdim; r += width) {
-        float acc = oc[group * a.vdim + r] * corr;
+    // one text for both would cost the large CTAs 8 to 25 % at long contexts
+    if constexpr (THREADS == kGpThreads) {
+      if (group < groups)
+        for (int r = column; r < a.vdim; r += width) {
+          float acc = oc[group * a.vdim + r] * corr;
 #pragma unroll 8
-        for (int j = group; j < n; j += groups)
+          for (int j = group; j < n; j += groups)
+            acc = fmaf(p[j], to_f32<T>(static_cast<const T*>(a.v_cache)[key_row[j] * a.v_ld + r]), acc);
+          oc[group * a.vdim + r] = acc;
+        }
+    } else {
+      for (int i = threadIdx.x; i < groups * a.vdim; i += THREADS) {
+        const int own = i / a.vdim, r = i % a.vdim;
+        float acc = oc[i] * corr;
+        for (int j = own; j < n; j += groups)
           acc = fmaf(p[j], to_f32<T>(static_cast<const T*>(a.v_cache)[key_row[j] * a.v_ld + r]), acc);
-        oc[group * a.vdim + r] = acc;
+        oc[i] = acc;
       }
+    }
   }
   __syncthreads();
   const float inv = (a.gates ? a.gates[t * a.heads + h] : 1.0f) / l;
@@ -724,7 +737,7 @@ grouped_plain_kernel(const GroupedAttn a) {
     for (int i = 0; i < groups; ++i) s += oc[i * a.vdim + r];
     return s * inv;
   };
-  for (int r = threadIdx.x * 2; r < a.vdim; r += kGpThreads * 2) {
+  for (int r = threadIdx.x * 2; r < a.vdim; r += THREADS * 2) {
     float u = total(r), v = r + 1 < a.vdim ? total(r + 1) : 0.f;
     a.turn_back(pos, r, u, v);
     dst[r] = from_f32<T>(u);
@@ -935,6 +948,14 @@ static GroupedAttn attn_args(const bcg_stack* m, const bcg_layer* l, const bcg_s
   return a;
 }
 
+template <typename T, int THREADS>
+static int launch_plain(const GroupedAttn& a, int n, cudaStream_t st) {
+  const int sm = (a.dim + plain_groups(a.dim, a.vdim) * a.vdim + kGpKeys) * 4;
+  BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_plain_kernel<T, THREADS>), 64 * 1024));
+  BCG_CUDA_CHECK(launch_k(grouped_plain_kernel<T, THREADS>, dim3(n, a.heads), dim3(THREADS), sm, st, a));
+  return BCG_OK;
+}
+
 // Tiles of 32 tokens or a CTA per token and head?  A tile walks the contexts of its sequences one behind another, where a token's CTA
 // has its own; over the same context a tile takes 2.9 times as long as a token's CTA.  Both have two CTAs per SM.  16 heads of 128,
 // contexts of 1,500, tiles / tokens: 1 x 64 tokens 213 / 333 us, 1 x 32 211 / 147, 8 x 16 327 / 662, 8 x 8 630 / 341, 8 x 3 1224 / 130.
@@ -957,16 +978,14 @@ static int grouped_plain(const bcg_stack* m, const bcg_layer* l, const bcg_stack
     BCG_CUDA_CHECK(launch_k(grouped_tile_kernel, dim3((n + kGtQueries - 1) / kGtQueries, l->heads), dim3(kGtThreads), kGtSmem, st, a, n));
     return BCG_OK;
   }
-  const int sm = (l->dim + plain_groups(l->dim, l->vdim) * l->vdim + kGpKeys) * 4;
-  const dim3 grid(n, l->heads);
-  if (m->act_dtype == BCG_DT_F32) {
-    BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_plain_kernel<float>), 64 * 1024));
-    BCG_CUDA_CHECK(launch_k(grouped_plain_kernel<float>, grid, dim3(kGpThreads), sm, st, a));
-  } else {
-    BCG_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_plain_kernel<__nv_bfloat16>), 64 * 1024));
-    BCG_CUDA_CHECK(launch_k(grouped_plain_kernel<__nv_bfloat16>, grid, dim3(kGpThreads), sm, st, a));
-  }
-  return BCG_OK;
+  // A bound on the keys of a token: the context of single tokens is known, and a window without pooled blocks.  Up to 32 keys, in more
+  // CTAs than are resident, small ones are faster (64 rows of 16 heads of 128 at one key 18.7 -> 8.3 us, at 16 keys 22.8 -> 10.5); at 410
+  // keys they would take 199 us for 110, and heads of 264 and 300 columns 18.5 for 14.8 at 16 keys.
+  long long keys = rows || b->n_tiles == 0 ? b->max_context : 1ll << 40;
+  if (l->window > 0 && l->pool == 0 && l->window < keys) keys = l->window;
+  const bool small = keys <= 32 && l->dim + l->vdim <= 256 && static_cast<long long>(n) * l->heads > 2 * num_sms();
+  if (m->act_dtype == BCG_DT_F32) return small ? launch_plain<float, kGpShort>(a, n, st) : launch_plain<float, kGpThreads>(a, n, st);
+  return small ? launch_plain<__nv_bfloat16, kGpShort>(a, n, st) : launch_plain<__nv_bfloat16, kGpThreads>(a, n, st);
 }
 
 // ------------------------------------------------------------------------------------------- decode

@@ -164,6 +164,19 @@ def test_grouped_attention_fp32_of_many_tokens(size, window):
     _check(a, _seqs(a, ((300, 200), (40, 21), (64, 1), (9, 3), (150, 150), (65, 64), (73, 73)), window), 3e-6)
 
 
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("size", ["plain", "usual", "odd-group", "huge"])
+def test_single_tokens_of_short_contexts_in_large_batches(size, dtype):
+    """Contexts of up to 32 keys in CTAs of 128 threads (many rows) and of 512 (one row): the same bits, at the edge too."""
+    a = Attention(size, 0, dtype, tokens=6400, rows=200, kv_pages=400)
+    for n in (1, 17, 32):
+        seqs = _seqs(a, [(max(1, n - i % 3), 1) for i in range(200)], n)
+        many, _ = _check(a, seqs, DT[dtype][2] if dtype == "float32" else 2e-2, mode=1)
+        for i in (0, 1, 199):
+            one, _ = a.run([seqs[i]], 1)
+            assert torch.equal(one[0], many[i])
+
+
 @pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
 @pytest.mark.parametrize("window", [0, 17])
 def test_values_that_are_not_finite_reach_only_the_tokens_that_see_them(value, window):
