@@ -359,13 +359,6 @@ gemm2sm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   if (warp == 1) tmem_dealloc_2sm(tmem_base, k2TmemCols);
 }
 
-static int pairs_of_sms() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms / 2;
-}
-
 // the last column tile may be partial (the epilogue stores 32 columns at a time), where that wastes little
 static bool for_pairs(int M, int N) {
   const int idle = (N + k2BlockN - 1) / k2BlockN * k2BlockN - N;
@@ -382,7 +375,7 @@ static bool for_pairs(int M, int N) {
 // take 512), slabs written and read at about 4 KB per clock.  At most `room` floats of output.
 int gemm_long_splits(int M, int N, int K, long long room) {
   if (!for_pairs(M, N)) return 1;
-  const int tiles = (M + 255) / 256 * ((N + k2BlockN - 1) / k2BlockN), kb = (K + k2BlockK - 1) / k2BlockK, pairs = pairs_of_sms();
+  const int tiles = (M + 255) / 256 * ((N + k2BlockN - 1) / k2BlockN), kb = (K + k2BlockK - 1) / k2BlockK, pairs = num_sms() / 2;
   const double slab = static_cast<double>(M) * N * 8.0 / 4096.0;
   int best = 1;
   double least = 0.0;
@@ -435,7 +428,7 @@ int gemm2sm_bf16_tn(const void* X, const void* W, void* out, int M, int N, int K
   if ((rc = make_tmap_bf16_sw128(&tma, X, M, K, ldx, k2BlockM)) != BCG_OK) return rc;
   if ((rc = make_tmap_bf16_sw128(&tmb, W, N, K, ldw, k2BlockN / 2)) != BCG_OK) return rc;
 
-  int clusters = pairs_of_sms();
+  int clusters = num_sms() / 2;
   const int total = a.tiles_m * a.tiles_n * a.splits;
   if (clusters > total) clusters = total;
   if (stages != 6) {

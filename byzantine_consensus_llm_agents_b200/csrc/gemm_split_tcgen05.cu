@@ -371,7 +371,8 @@ int gemm_f32(const float* X, const void* W, float* out, int M, int N, int K, lon
   a.vec_out = (reinterpret_cast<uintptr_t>(out) % 16 == 0 && ldo % 4 == 0) ? 1 : 0;
   // Rounds of one CTA per SM; a narrow tile takes a little more than half the time of a wide one (the conversion is the same)
   const long long wide = static_cast<long long>(a.tiles_m) * ((N + 127) / 128), narrow = static_cast<long long>(a.tiles_m) * ((N + 31) / 32);
-  return (wide + 147) / 148 * 2 > (narrow + 147) / 148 ? launch_split<32>(W, a, ldw, st) : launch_split<128>(W, a, ldw, st);
+  const int sms = num_sms();
+  return (wide + sms - 1) / sms * 2 > (narrow + sms - 1) / sms ? launch_split<32>(W, a, ldw, st) : launch_split<128>(W, a, ldw, st);
 }
 
 }  // namespace bcg

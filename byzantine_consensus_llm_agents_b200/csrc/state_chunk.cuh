@@ -12,6 +12,7 @@
 #pragma once
 #include <type_traits>
 
+#include "kernels.h"
 #include "state_rows.cuh"
 
 namespace bcg {
@@ -485,7 +486,7 @@ static int launch_segments(const typename RULE::Args& a, dim3 grid, cudaStream_t
 template <int NP, class RULE>
 static int launch_chunks(const typename RULE::Args& a, dim3 grid, int n_tokens, int n_seqs, cudaStream_t st) {
   if constexpr (!RULE::kNormalized) {
-    const long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z, slots = 148ll * ChCfg<NP, RULE>::kCtasPerSm;
+    const long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z, slots = static_cast<long long>(num_sms()) * ChCfg<NP, RULE>::kCtasPerSm;
     const int chunks = n_tokens / n_seqs / kChTok;
     if (ctas * 4 <= slots && chunks >= 8) return launch_segments<NP, RULE, 4>(a, grid, st);
     if (ctas * 2 <= slots && chunks >= 4) return launch_segments<NP, RULE, 2>(a, grid, st);
