@@ -156,6 +156,20 @@ def test_gemm_long_launches_on_pairs_and_single_sms(N, K, epi):
         assert torch.equal(out, want[:M]), M
 
 
+@pytest.mark.parametrize("M,N,K,splits", [(10, 256, 128, 8), (300, 256, 128, 8), (300, 1024, 72, 3), (700, 4096, 640, 7), (130, 2048, 512, 3),
+                                          (1000, 512, 64, 2)])
+def test_gemm_more_parts_than_k_blocks(M, N, K, splits):
+    """Parts of K for launches of few and many rows; with more parts than k-blocks the first ones are the product and the others are
+    left alone."""
+    x, w = _rand_bf16(M, K, seed=51), _rand_bf16(N, K, scale=0.05, seed=52)
+    out = torch.full((splits, M, N), 7.0, dtype=torch.float32, device=DEV)
+    L.gemm(x, w, out, L.EPI_F32, splits=splits)
+    used = min(splits, (K + 63) // 64)
+    err = (out[:used].double().sum(0) - x.double() @ w.double().T).abs().max().item()
+    assert err <= 1e-4 * math.sqrt(K) + 1e-5, err
+    assert (out[used:] == 7.0).all()
+
+
 def test_gemm_rejects_bad_args():
     x = _rand_bf16(4, 64)
     w = _rand_bf16(128, 64)

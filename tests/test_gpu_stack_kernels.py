@@ -351,6 +351,14 @@ def test_gemm_any_aligned_rows(M, N, K):
         assert (out[:, N:] == 7.0).all()
 
 
+# The same with more k-blocks than the kernel has stages and accumulators, an even and an odd count of them, in both widths of tile; and
+# fewer inputs than a k-block has.
+@pytest.mark.parametrize("M,N,K", [(300, 2500, 1032), (260, 12320, 520), (300, 2500, 2048), (820, 2048, 1416), (40, 1030, 1480), (129, 70, 2056),
+                                   (6, 130, 8), (40, 2048, 24), (300, 2500, 56)])
+def test_gemm_any_aligned_rows_of_many_and_few_inputs(M, N, K):
+    test_gemm_any_aligned_rows(M, N, K)
+
+
 def test_gemm_any_keeps_infinities_and_nans():
     g = gen(0)
     x, w = torch.randn(40, 512, generator=g), torch.randn(64, 512, generator=g).bfloat16()
@@ -406,3 +414,25 @@ def test_sandwich_norm_of_wide_long_launches(T, d, parts):
 @pytest.mark.parametrize("T,ff,parts", [(129, 4096, 1), (130, 7424, 1), (129, 16384, 1), (129, 16388, 1), (129, 4100, 2)])
 def test_poly_norm_of_long_launches(dtype, T, ff, parts):
     test_poly_norm(dtype, T, ff, parts)
+
+
+@pytest.mark.parametrize("T,d,parts", [(6, 2048, 2), (150, 2048, 1), (140, 4096, 2), (150, 8192, 1), (6, 8196, 1)])
+@pytest.mark.parametrize("value", [math.inf, math.nan])
+def test_norms_keep_rows_apart(T, d, parts, value):
+    """A row with an infinite or NaN summand, its neighbours as without it: PolyNorm and the sandwich norm, rows over clusters, in
+    registers and staged."""
+    lib, g = L.load(), gen(T + d)
+    x, y = dev(torch.randn(T, d, generator=g)), dev(torch.randn(parts, T, d, generator=g))
+    w, coef = dev(torch.randn(d, generator=g)), torch.tensor([0.9, -0.5, 0.3, 0.2], device="cuda")
+
+    def run(y):
+        res, xn, act = x.clone(), torch.zeros(T, d, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, d, dtype=torch.bfloat16, device="cuda")
+        L.check(lib.bcg_sandwich_norm(res.data_ptr(), y.data_ptr(), parts, T * d, w.data_ptr(), w.data_ptr(), xn.data_ptr(), L.DT_BF16, T, d,
+                                      1e-5, L.stream_ptr()))
+        L.check(lib.bcg_poly_norm(y.data_ptr(), parts, T * d, coef.data_ptr(), act.data_ptr(), L.DT_BF16, T, d, 1e-5, L.stream_ptr()))
+        return res, xn, act
+    clean = run(y)
+    y[parts - 1, 2, d - 3] = value
+    rest = [t for t in range(T) if t != 2]
+    for a, b in zip(run(y), clean):
+        assert torch.equal(a[rest], b[rest]) and not torch.isfinite(a[2]).all()
