@@ -3,12 +3,12 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
 
-Workload (BASELINE.json configs[2], the one `metric` is quoted on): Qwen3-14B architecture,
+Workload (the one `metric` is quoted on): Qwen3-14B architecture,
 random-init bf16 weights, 8 honest + 2 Byzantine agents.  One STEP = one game round's agent step:
 every agent's *decide* call (T=0.5, <=300 tokens) and *vote* call (T=0.3, <=200 tokens) through
 `VLLMAgent.batch_generate_json`, with the reference's retry schedule (main.py:256-478: up to 3
 batched attempts per phase; with random-init weights every attempt runs to the token limit and
-fails validation — the "retry storm" of SURVEY.md F7).  Prompts are the (system, user, schema)
+fails validation — the "retry storm").  Prompts are the (system, user, schema)
 triples the unmodified reference builds in steady-state rounds 6.. (tests/golden/
 bench_prompts_*.json.gz, produced by oracle/tools/make_bench_prompts.py); each step uses the next
 recorded round, so only what really repeats in a game (per-agent system prompts, identical retry
@@ -31,7 +31,7 @@ Printed JSON (one line, rank 0):
   ranks   per-rank device / wall seconds of the faithful region (value uses the max, as the
           contract says; value_mean_over_ranks is beside it)
   single_game (N > 1)  ONE game whose rows are sharded over the N replicas (dp.run_sharded): the
-          latency half of SURVEY.md §8e; `value` above is the aggregate half (one game per replica)
+          latency half; `value` above is the aggregate half (one game per replica)
 """
 from __future__ import annotations
 
@@ -400,7 +400,7 @@ def main():
     if a.impl == "reference":
         if rank != 0:
             return
-        # The reference's own engine (vLLM) cannot run here (SURVEY.md F3; BASELINE.md §2); its CPU
+        # The reference's own engine (vLLM) cannot run here; its CPU
         # path is the oracle port, timed on the host cores.
         # One STEP of this arm = one bounded sample (about 3-4 s of CPU work: 1,024-token prefill + 48
         # guided decode steps on a 2-layer full-width slice); W warm-up samples, then exactly K timed
@@ -531,7 +531,7 @@ def main():
                                                  for k, v in fixed_phases.items()},
                  "schedule": f"{MAX_RETRIES} batched attempts per phase, all {n_agents} rows forced to max_tokens"}
 
-    # ---- ONE game, rows sharded over the replicas (latency half of SURVEY.md §8e)
+    # ---- ONE game, rows sharded over the replicas (latency half)
     single = None
     if world > 1 and a.tp == 1 and a.single_game_steps > 0:
         engine.reset_prefix_cache()
@@ -556,7 +556,7 @@ def main():
     if rank == 0:
         cfg = engine.cfg
         gen, steps = d["generated_tokens"], d["decode_steps"]
-        # whole-step decode roofline: W + sum_rows S*KVB per step (SURVEY.md §8d)
+        # whole-step decode roofline: W + sum_rows S*KVB per step
         avg_rows = d["generated_tokens"] / max(1, d["decode_steps"])
         avg_ctx = (d["prompt_tokens"] / max(1, d["prompts"])) + 0.5 * (gen / max(1, d["prompts"]))
         # per GPU: under TP every rank streams 1/tp of the weights and of the KV heads

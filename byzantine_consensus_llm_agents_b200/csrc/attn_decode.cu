@@ -1,4 +1,4 @@
-// Batched decode attention over the paged bf16 KV cache (SURVEY.md §2.1 row K8):
+// Batched decode attention over the paged bf16 KV cache:
 // one query token per row, GQA (the q-heads that share a KV head share each KV load),
 // HBM-bound.  Work is split along the context in FIXED 256-token chunks (16 pages), so a
 // row's arithmetic — chunk boundaries and the order partial results are merged in —

@@ -1,5 +1,5 @@
 // Fused causal prefill attention over the paged bf16 KV cache with a cached-prefix offset
-// (SURVEY.md §2.1 row K7; stands in for the FlashInfer `fmhaSm100a...PagedKv...Context` kernels
+// (stands in for the FlashInfer `fmhaSm100a...PagedKv...Context` kernels
 // vLLM dispatches on sm_100).  New tokens of every sequence are concatenated ("ragged") in q;
 // K/V for *all* positions — the reused prefix pages and the pages just written by
 // qknorm_rope_kvwrite — are read through the block table, so prefix-cache hits and cold

@@ -132,8 +132,8 @@ struct StateTile {
   // from shared memory, is what the loop is bound by when CPT is small.)  Returns the output of column col + output_of(lane).
   //
   // The sums over a column's eight row groups are halved on the way: a lane sends one half of its values and keeps the other, so
-  // that 2 CPT values take 2 CPT - 1 exchanges (or three), and CPT more bring u^T S back to every lane; with sums complete in every
-  // lane there were 6 CPT of them (16 heads of eight prompts up to 1,843 tokens: 1267 -> 1194 us).
+  // that 2 CPT values take seven, four or three exchanges (CPT 4, 2, 1), and CPT more bring u^T S back to every lane; with sums complete
+  // in every lane there were 6 CPT of them (16 heads of eight prompts up to 1,808 tokens: 1267 -> 1194 us).
   __device__ __forceinline__ float token(const float* op, int pitch, const float* sc, int rg, int col) {
     constexpr bool kKeep = kQ <= 4;       // k stays in registers between its two uses
     const int lane = threadIdx.x & 31;

@@ -370,9 +370,10 @@ static bool for_pairs(int M, int N) {
 // 951 rows 31.5 / 31.5 / 37.7 and 74.4 / 76.3 / 78.4, so that they stay whole.
 //
 // How many parts of K the fp32 product of a long launch is best cut into, where the consumer adds slabs (in layer stacks; rows of
-// dense models must not depend on their launch): tiles that leave pairs of
-// SMs idle in the last round cost more than the slabs do.  Clocks: 520 per k-block and round (measured over 12 k rows; the MMAs
-// take 512), slabs written and read at about 4 KB per clock.  At most `room` floats of output.
+// dense models must not depend on their launch): tiles that leave pairs of SMs idle in the last round cost more than the slabs do.
+// Clocks: 520 per k-block and round (measured over 12 k rows; the MMAs take 512), slabs written and read at about 4 KB per clock.  At most
+// `room` floats of output.  With the norm behind it, against every other count of parts at 2,048 and 4,096 columns, 2,048 to 23,680
+// inputs and 129 to 3,000 rows: at most 13 % off the best, and never slower than whole.
 int gemm_long_splits(int M, int N, int K, long long room) {
   if (!for_pairs(M, N)) return 1;
   const int tiles = (M + 255) / 256 * ((N + k2BlockN - 1) / k2BlockN), kb = (K + k2BlockK - 1) / k2BlockK, pairs = num_sms() / 2;

@@ -1,6 +1,6 @@
 // Dense projection GEMM for the agent-step engine:  Y[M,N] = X[M,K] · W[N,K]^T
 // (bf16 in, fp32 accumulate in TMEM).  Replaces the cuBLAS F.linear calls the
-// reference reaches through vLLM (SURVEY.md §2.1 rows K3, K9, K10, K11, K12).
+// reference reaches through vLLM.
 //
 // One persistent, warp-specialised kernel serves both regimes:
 //   * prefill (M large, tensor-bound): A-operand = activations (128-row tiles on the

@@ -1,4 +1,4 @@
-// Memory-bound glue kernels of the decoder layer (SURVEY.md §2.1 rows K1, K2, K4, K5, K6):
+// Memory-bound glue kernels of the decoder layer:
 //   embed_rmsnorm        K1+K2 : h = E[ids]; xn = rmsnorm(h) * w
 //   add_rmsnorm          K2    : h += delta (bf16, or fp32 split-K partials summed in fixed order);
 //                                xn = rmsnorm(h) * w
@@ -8,7 +8,7 @@
 // The residual stream is kept in fp32 (tighter against the fp32 CPU forward that is the
 // oracle); every row is computed independently of the batch it is in (batch-invariant).
 // Arithmetic follows transformers' Qwen3RMSNorm / apply_rotary_pos_emb in fp32
-// (modeling_qwen3.py:50-64,86-148 as cited in SURVEY.md §8c).
+// (transformers' modeling_qwen3.py:50-64,86-148).
 #include <cooperative_groups.h>
 #include <stdlib.h>
 

@@ -1,11 +1,11 @@
-// Grammar-constrained sampler (SURVEY.md §2.1 rows K13-K15) fused with the per-row decode
+// Grammar-constrained sampler fused with the per-row decode
 // bookkeeping, so the decode loop never returns to the host between tokens.
 //
 // One thread-block CLUSTER (8 CTAs x 512 threads) per row: each CTA scans 1/8 of the
 // vocabulary with 128-bit loads, applies the token bitmask of the row's DFA state,
 // computes the race score, reduces (score, index) with warp shuffles, and the eight CTA
-// winners meet in CTA 0's shared memory through DSMEM.  (north_star words this as a
-// "warp-per-row" kernel; at V = 151,936 and ~10 rows a single warp per row would leave
+// winners meet in CTA 0's shared memory through DSMEM.  (A warp per row would
+// do; at V = 151,936 and ~10 rows that would leave
 // the chip idle for ~100 us per token, so the row is spread over a cluster instead —
 // same fusion, same arithmetic.)
 //

@@ -121,7 +121,7 @@ __device__ __forceinline__ void chunk_matrix(const RULE& rule, uint32_t sB, uint
 // SEG > 1 (rules without normalizer): few heads and sequences leave most of the chip idle while each walks its chunks one by one.
 // A cluster of SEG CTAs then shares a sequence's chunks: each first runs its part's state alone, from zero (a state's update, less
 // than half of a chunk's work), the states are handed on from CTA to CTA, S <- (what the part adds) + (its decay) S, and with the
-// state that comes in each runs its part whole.  64 heads, launches of 2,048 and of 951 tokens: 116 -> 63 us on average.
+// state that comes in each runs its part whole.  64 heads, launches of 2,048 and of 1,092 tokens: 116 -> 63 us on average.
 template <int NP, class RULE, int SEG>
 __global__ void __launch_bounds__(kChThreads, ChCfg<NP, RULE>::kCtasPerSm)
 chunk_kernel(const typename RULE::Args a) {

@@ -1,7 +1,7 @@
 // Tensor-parallel plumbing: one NCCL communicator per process (one process per GPU), used by the
 // model steps for the two all-reduces per layer (after the row-parallel o and down projections)
 // and the all-gather of vocab-parallel logits — the collectives vLLM issues for the reference when
-// `tensor_parallel_size > 1` (vllm_agent.py:131,141-142; SURVEY.md §2.1 C1-C3).
+// `tensor_parallel_size > 1` (vllm_agent.py:131,141-142).
 // libnccl is the one PyTorch already loaded; it is resolved with dlopen so the library has no
 // link-time dependency on it and single-GPU users never touch it.
 #include <dlfcn.h>

@@ -1,4 +1,4 @@
-"""Data parallelism over model replicas (SURVEY.md §8e): one process per GPU, full weights each.
+"""Data parallelism over model replicas: one process per GPU, full weights each.
 
 Two independent things shard with no data-path collective:
   * ROWS of one `batch_generate_json` call — every (agent, phase) generation depends only on its

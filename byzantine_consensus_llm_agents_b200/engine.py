@@ -7,7 +7,7 @@ whole model forward, paged attention, grammar-masked sampling and ALL per-token 
 after prefill the decode loop is a CUDA graph replayed once per token with no host round trip;
 the host only polls a single counter every few steps to stop early.
 
-Differences from the engine the reference reaches (deliberate, SURVEY.md F4/F5):
+Differences from the engine the reference reaches (deliberate):
   * every row of a call is decoded together, each with its own grammar (the reference falls
     back to one-prompt-at-a-time when schemas differ, vllm_agent.py:417-455) and without the
     `max_num_seqs=4` cap (config.py:38) — per-row results are batch-invariant, so this changes

@@ -1,7 +1,7 @@
-"""Game-level data parallelism: many seeded games per box, one engine
+"""Data parallelism of whole games: many seeded games per box, one engine
 replica per GPU, results gathered into one table.
 
-Whole games are the unit that really scales with GPUs (§8e: inside one game every replica would
+Whole games are the unit that really scales with GPUs (inside one game every replica would
 re-read the same weights each decode step).  The reference offers `run_simulation(n_agents,
 max_rounds, model_name, byzantine_count, byzantine_awareness) -> {"metrics": stats}`
 (main.py:1073-1141) for batch experiments but no driver around it; this module is that driver:

@@ -1,4 +1,4 @@
-"""JSON-schema -> byte-level DFA -> token-level mask tables (SURVEY.md §2.1 K13, §3.5).
+"""JSON-schema -> byte-level DFA -> token-level mask tables.
 
 The reference asks vLLM for `GuidedDecodingParams(json=schema)` (vllm_agent.py:318, 423);
 vLLM's default backend compiles the schema with xgrammar (`any_whitespace=True`) and, every

@@ -1,7 +1,7 @@
 """Model descriptions and weight packing for the engine.
 
 Architectures are the ones the reference's MODEL_PRESETS name (config.py:20-25) with the
-dimensions of SURVEY.md §8d.  Weights are random-init (there are no checkpoints offline):
+dimensions of the published models.  Weights are random-init (there are no checkpoints offline):
 N(0, 0.02) linears/embeddings, norm weights 1 — transformers' default init — either taken from
 a transformers state_dict (parity tests: same values as the CPU oracle) or generated directly
 on the GPU (bench).  All matrices are bf16; norm weights and the RoPE table are fp32.
@@ -61,7 +61,7 @@ class ModelConfig:
         return 2 * per
 
     def decode_weight_bytes(self) -> int:
-        """bf16 bytes streamed per decode step: all layer matrices + lm_head (SURVEY §8d col 9)."""
+        """bf16 bytes streamed per decode step: all layer matrices + lm_head."""
         return self.n_layers * self.layer_weight_bytes() + 2 * self.vocab * self.d_model
 
     def prefill_gemm_flops_per_token(self) -> int:

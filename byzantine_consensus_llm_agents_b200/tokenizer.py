@@ -1,4 +1,4 @@
-"""Deterministic synthetic tokenizer (SURVEY.md F9 / H6).
+"""Deterministic synthetic tokenizer.
 
 The reference lets vLLM load the HuggingFace tokenizer of the model it names
 (vllm_agent.py:126-144); no tokenizer files exist offline, so the engine — and the CPU oracle,
@@ -12,7 +12,7 @@ geometry:
                             decodable and visible to the grammar mask): words, digits,
                             punctuation/JSON fragments, whitespace runs, UTF-8 characters and
                             partial UTF-8 sequences — so masks have realistic density and tokens
-                            straddle grammar boundaries (SURVEY.md H4)
+                            straddle grammar boundaries
   * qwen3 family:  26 special tokens at n_regular.. with <|endoftext|>, <|im_start|>,
                    <|im_end|> first (151643/4/5 at the full 151,936 vocabulary); ids above the
                    last special token up to the model's vocab are unused padding, as in Qwen.

@@ -236,7 +236,7 @@ class VLLMAgent:
 
     @staticmethod
     def _check_sampling(top_p: float, kwargs: Dict[str, Any]) -> None:
-        # The reference never sets top_p / extra sampling options (SURVEY.md a13); refusing them
+        # The reference never sets top_p / extra sampling options; refusing them
         # is better than silently sampling from a different distribution.
         if top_p != 1.0 or kwargs:
             raise NotImplementedError("only temperature / max_tokens sampling is implemented "

@@ -6,7 +6,7 @@
  * `vllm.LLM.generate` (vllm_agent.py:195,331,430,502).  The Python class in
  * byzantine_consensus_llm_agents_b200/vllm_agent.py replaces that module one-for-one; the
  * functions below are what that class binds (ctypes) in place of the third-party engine's
- * CUDA ops.  Each entry cites the engine op it stands in for (SURVEY.md §2.1 K1..K15).
+ * CUDA ops.  Each entry cites the engine op it stands in for.
  *
  * Conventions: plain pointers and sizes only; every pointer is DEVICE memory owned by the
  * caller unless the comment says host; `stream` is a cudaStream_t passed as void*; no entry
@@ -46,7 +46,7 @@ const char* bcg_last_error(void);
 /* Y[M,N] = X[M,K] · W[N,K]^T, bf16 inputs, fp32 accumulation on tcgen05 tensor cores with
  * TMEM accumulators and TMA-fed operands.  Stands in for the cuBLAS `F.linear` calls of
  * qkv_proj / o_proj / gate_up_proj (+ `_C.silu_and_mul`) / down_proj / lm_head
- * (vLLM model_executor/models/qwen3.py:145-162,216-236; SURVEY.md K3, K9-K12).
+ * (vLLM model_executor/models/qwen3.py:145-162,216-236).
  * M <= 128 selects the weight-streaming (swap-AB, optional split-K) decode path.
  * ldx, ldw, ld_out are row pitches in elements.  splits > 1 requires BCG_EPI_F32 and an
  * `out` buffer of splits*M*ld_out floats; the consumer sums the partials in index order. */
@@ -83,7 +83,7 @@ int bcg_gemm_bf16_tn_fused(const void* X, const void* W, void* out, int M, int N
 int bcg_gemm_splits_for(int M, int N, int K);
 
 /* residual[t,:] = embed[ids[t],:] (fp32); xn[t,:] = rmsnorm(residual[t,:]) * w  (bf16).
- * Stands in for `F.embedding` + `_C.rms_norm` (SURVEY.md K1, K2). */
+ * Stands in for `F.embedding` + `_C.rms_norm`. */
 int bcg_embed_rmsnorm(const int* ids, const void* embed, const float* w, float* residual, void* xn,
                       int T, int d, float eps, void* stream);
 
@@ -91,7 +91,7 @@ int bcg_embed_rmsnorm(const int* ids, const void* embed, const float* w, float* 
  * n_partials fp32 slabs [T,d] spaced partial_stride floats apart, summed in index order;
  * delta may be NULL.  If src_rows != NULL, output row i is computed from row src_rows[i] and
  * residual is not written (last-token gather in front of lm_head).
- * Stands in for `_C.fused_add_rms_norm` (SURVEY.md K2). */
+ * Stands in for `_C.fused_add_rms_norm`. */
 int bcg_add_rmsnorm(float* residual, const void* delta, int delta_is_f32, int n_partials,
                     long long partial_stride, const float* w, void* xn, const int* src_rows, int T,
                     int d, float eps, void* stream);
@@ -102,7 +102,7 @@ int bcg_add_rmsnorm(float* residual, const void* delta, int delta_is_f32, int n_
  * bcg_gemm_fusion.scale_sumsq with scale_tiles = 8, scale_d = d to the projection that reads xn.
  * T <= 128.  Takes the row-wide reduction (a cluster barrier and a DSMEM exchange in
  * bcg_add_rmsnorm) off the critical path between two GEMMs.  Stands in for the same vllm op,
- * `_C.fused_add_rms_norm` (SURVEY.md K2), with its last multiply moved into the next projection. */
+ * `_C.fused_add_rms_norm`, with its last multiply moved into the next projection. */
 int bcg_add_norm_stats(float* residual, const void* delta, int delta_is_f32, int n_partials,
                        long long partial_stride, const float* w, void* xn, float* sumsq, int T, int d,
                        void* stream);
@@ -112,8 +112,7 @@ int bcg_add_norm_stats(float* residual, const void* delta, int delta_is_f32, int
  * paged cache at slot_map[t] (slot = page*page_size + offset; negative = skip).
  * qkv is bf16 [T, ld_qkv] or fp32 split-K partials.  head_dim is 128.
  * KV cache layout (one layer): [page][2][n_kv_heads][page_size][128] bf16.
- * Stands in for `_C.rms_norm` on heads + `_C.rotary_embedding` + `reshape_and_cache_flash`
- * (SURVEY.md K4-K6). */
+ * Stands in for `_C.rms_norm` on heads + `_C.rotary_embedding` + `reshape_and_cache_flash`. */
 int bcg_qknorm_rope_kvwrite(const void* qkv, int qkv_is_f32, int n_partials,
                             long long partial_stride, long long ld_qkv, const float* q_norm_w,
                             const float* k_norm_w, const float* cos_sin, const int* positions,
@@ -132,7 +131,7 @@ int bcg_swiglu_reduce(const float* partials, int n_partials, long long partial_s
  * their own: partial results written by a call of another shape must never land on them);
  * max_splits >= ceil(max seq_len / 256) — a longer row makes the kernel trap (the launch fails with
  * a CUDA error) rather than leave its output unwritten.
- * Stands in for the FlashInfer paged decode kernel vLLM dispatches on sm_100 (SURVEY.md K8). */
+ * Stands in for the FlashInfer paged decode kernel vLLM dispatches on sm_100. */
 int bcg_decode_attn_paged(const void* q, const void* kv_cache, const int* block_table,
                           int max_blocks_per_seq, const int* seq_lens, void* out, float* scratch_o,
                           float* scratch_ml, int* chunk_counters, int B, int n_heads, int n_kv_heads,
@@ -144,7 +143,7 @@ int bcg_decode_attn_paged(const void* q, const void* kv_cache, const int* block_
  * itself; the CTA of a row's last chunk also builds the new token's K/V row, writes it to
  * kv_cache (slot_map[b], negative = skip) and patches it into the page it streamed in.  Stands in
  * for the same vLLM ops as the two entry points it replaces (`_C.rotary_embedding`,
- * `reshape_and_cache_flash`, FlashInfer paged decode; SURVEY.md K4-K6, K8).  Other arguments as
+ * `reshape_and_cache_flash`, FlashInfer paged decode).  Other arguments as
  * for bcg_decode_attn_paged. */
 int bcg_decode_attn_paged_qkv(const float* qkv, int n_partials, long long partial_stride,
                               long long ld_qkv, const float* q_norm_w, const float* k_norm_w,
@@ -179,7 +178,7 @@ int bcg_decode_attn_paged_static(const void* q, const void* kv_cache, const int*
  * fetched by TMA through tensor maps over the caller's q buffer and KV cache.  Every KV page a tile
  * reads (pages 0 .. ceil((position + rows) / 16) - 1 of its sequence's block-table row) must hold
  * finite values, including the unwritten tail of the last page (zero-initialise the cache).
- * Stands in for the FlashInfer paged prefill kernel (SURVEY.md K7). */
+ * Stands in for the FlashInfer paged prefill kernel. */
 int bcg_prefill_attn_paged(const void* q, const void* kv_cache, const int* block_table,
                            int max_blocks_per_seq, const int* tile_info, int n_tiles, void* out,
                            int n_q_rows, int n_heads, int n_kv_heads, int page_size, float scale,
@@ -193,7 +192,7 @@ int bcg_prefill_attn_paged(const void* q, const void* kv_cache, const int* block
  * bytes; appends the token; updates next_ids / positions / seq_lens / slot_map so the next
  * decode step needs no host round-trip.
  * Stands in for xgrammar `apply_token_bitmask_inplace` + vLLM `Sampler` + the scheduler's
- * accept_token/stop bookkeeping (SURVEY.md K13-K15; vllm v1/sample/sampler.py:91,223-297,
+ * accept_token/stop bookkeeping (vllm v1/sample/sampler.py:91,223-297,
  * v1/sample/ops/topk_topp_sampler.py:395-416, v1/structured_output/backend_xgrammar.py:148-192). */
 typedef struct bcg_sampler_args {
   const float* logits;     /* [B, ld_logits]; or vocab-sharded, see shard_v */
@@ -232,7 +231,7 @@ typedef struct bcg_sampler_args {
    * logits[(i / shard_v) * shard_stride + b * shard_v + i % shard_v]; 0 = plain [B, ld_logits] */
   int shard_v;
   long long shard_stride;
-  /* vocab-parallel sampling without moving logits (tensor parallelism, SURVEY.md C2): tp_size > 1
+  /* vocab-parallel sampling without moving logits (tensor parallelism): tp_size > 1
    * means `logits` holds only this rank's shard — V tokens starting at token id vocab_base (a
    * multiple of 4; mask rows still span the whole vocabulary) — and the ranks trade one
    * (score, token id) candidate per row through the symmetric buffer (bcg_tp_symm_create / _open)
@@ -242,8 +241,8 @@ typedef struct bcg_sampler_args {
   int vocab_base;
 } bcg_sampler_args;
 
-/* Launches the sampler described above on `stream` (stands in for xgrammar's mask apply + vLLM's
- * Sampler + accept_token bookkeeping, SURVEY.md K13-K15).  `args` is a HOST struct of device pointers. */
+/* Launches the sampler described above on `stream` (Stands in for xgrammar's mask apply + vLLM's
+ * Sampler + accept_token bookkeeping).  `args` is a HOST struct of device pointers. */
 int bcg_mask_sample(const bcg_sampler_args* args, void* stream);
 
 /* Tensor parallelism (Qwen3-32B TP=8, Mistral-22B TP=2 in the reference's presets): one process per
@@ -252,7 +251,7 @@ int bcg_mask_sample(const bcg_sampler_args* args, void* stream);
  * steps then all-reduce the outputs of the row-parallel o / down projections (2 per layer); the
  * vocab-parallel logits stay sharded and the sampler exchanges one candidate per row, standing in
  * for vLLM's TP collectives
- * (vllm_agent.py:131,141-142; SURVEY.md C1-C3).  libnccl.so.2 is resolved at run time. */
+ * (vllm_agent.py:131,141-142).  libnccl.so.2 is resolved at run time. */
 int bcg_tp_unique_id(void* out_128_bytes /* host */);
 int bcg_tp_init(const void* id_128_bytes /* host */, int rank, int size);
 int bcg_tp_shutdown(void);
@@ -276,7 +275,7 @@ int bcg_tp_symm_open(const void* handles_size_x_64_bytes /* host */, int rank, i
  * (bit-identical on every rank), then residual += sum, xn = bf16(residual * w) and
  * sumsq[s * 128 + t] as bcg_add_norm_stats.  Collective: every rank of the replica must make the same
  * sequence of calls.  Stands in for vLLM's tensor_model_parallel_all_reduce after RowParallelLinear
- * + `_C.fused_add_rms_norm` (SURVEY.md C1, K2). */
+ * + `_C.fused_add_rms_norm`. */
 int bcg_tp_add_norm_stats(float* residual, const float* partials, int n_partials, long long partial_stride,
                           const float* w, void* xn, float* sumsq, int slot, long long region_floats, int T,
                           int d, void* stream);
@@ -342,7 +341,7 @@ int bcg_model_prefill(const bcg_model* m, const bcg_workspace* ws, const int* id
 int bcg_model_head(const bcg_model* m, const bcg_workspace* ws, const int* rows, int n, int row0, void* stream);
 /* One decode step for B rows: ids/positions/slot_map/seq_lens are the arrays bcg_mask_sample
  * maintains; logits land in ws->logits[0..B).  Stands in for one decode step of the same vLLM
- * forward (SURVEY.md a10).  flags: BCG_GEMM_PDL, plus how the residual add + RMSNorm between two
+ * forward.  flags: BCG_GEMM_PDL, plus how the residual add + RMSNorm between two
  * projections is executed on a single GPU (both variants need ws->row_sumsq / ws->tile_counters):
  *   default                   bcg_add_rmsnorm kernels (complete norm, then the projection)
  *   BCG_STEP_DEFERRED_NORM    bcg_add_norm_stats + 1/RMS applied in the next projection's epilogue
@@ -572,8 +571,9 @@ int bcg_stack_head(const bcg_stack* m, const bcg_stack_ws* ws, const int* rows, 
 
 /* The mechanisms one by one (what bcg_stack_step launches; the reference has no counterpart).
  * `in` arguments with n_partials slabs are fp32 split-K outputs added in index order. */
-/* out fp32 [M, ldo] = X [M, ldx] (act_dtype) * W bf16 [N, ldw]^T in fp32, any shape: on tensor cores where X is
- * fp32 and rows start on 16 bytes, on CUDA cores elsewhere. */
+/* out fp32 [M, ldo] = X [M, ldx] (act_dtype) * W bf16 [N, ldw]^T in fp32, any shape.  X fp32 with rows that start on 16
+ * bytes: more than four rows on tensor cores (X in three bf16 parts), up to four as FMAs; all else on CUDA cores.
+ * Infinities and NaNs come out as FMAs give them. */
 int bcg_gemm_any(const void* X, int x_dtype, const void* W, float* out, int M, int N, int K, long long ldx,
                  long long ldw, long long ldo, void* stream);
 /* No counterpart in the reference: residual += w_post ? rmsnorm(delta) * w_post : delta, then

@@ -3,7 +3,7 @@
 The model-forward oracle: transformers' own fp32 CPU implementation of the architectures the
 reference names (Qwen3ForCausalLM / MistralForCausalLM, transformers 5.5.0 —
 modeling_qwen3.py:50-64 RMSNorm, 70-83 MLP, 151-181 RoPE, 252-291 attention with per-head q/k
-norm before RoPE, 305-334 decoder layer), built from an explicit config (SURVEY.md §8d) with
+norm before RoPE, 305-334 decoder layer), built from an explicit config with
 `torch.manual_seed(seed)` and transformers' default init (N(0, 0.02), norm weights 1).
 Weights are rounded to bf16 values (kept in fp32 storage) so that oracle and engine hold
 IDENTICAL parameters; all arithmetic here is fp32.

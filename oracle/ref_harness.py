@@ -1,8 +1,8 @@
 """ORACLE (test infrastructure only — never imported by the product path).
 
 Runs the UNMODIFIED reference (`/root/reference/byzantine_consensus_game/*.py`) in this
-container by supplying the third-party `vllm` package it imports (cut line B2 of SURVEY.md
-§8b): `vllm.LLM`, `vllm.SamplingParams`, `vllm.sampling_params.GuidedDecodingParams`
+container by supplying the third-party `vllm` package it imports (the engine
+boundary): `vllm.LLM`, `vllm.SamplingParams`, `vllm.sampling_params.GuidedDecodingParams`
 (vllm_agent.py:13-14).  The shim forwards `LLM.generate(prompts, sampling_params)` to a
 pluggable backend and records every call, which is how the golden fixtures under
 tests/golden/ are produced (oracle/tools/*.py).

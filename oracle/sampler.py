@@ -10,7 +10,7 @@ CPU restatement of the sampler the reference reaches through vLLM, in numpy:
                                                      vllm/v1/sample/ops/topk_topp_sampler.py:129,395-416
 
 vLLM draws q from torch's global CUDA generator, which no other implementation can
-reproduce (SURVEY.md H5).  The engine therefore defines its own counter-based stream —
+reproduce.  The engine therefore defines its own counter-based stream —
 Philox4x32-10 keyed by a per-row seed, counter (i >> 2, step, 0, 0) — and evaluates the same
 exponential race in the log domain:
 

@@ -3,7 +3,7 @@
 Re-runs the fp32 CPU forward with only the bf16 roundings the engine performs (GEMM inputs xn /
 attn / act, q, k, v, P, final xn) switched on one at a time and all together.  Measured
 (wide-qwen3, 2 layers, d=1024): all roundings -> rms 0.0048, max 0.026 of a logit std 0.64; the
-GPU engine measures rms 0.004 — i.e. it sits on the rounding floor (DESIGN.md §6).
+GPU engine measures rms 0.004 — i.e. it sits on the rounding floor.
     python -m oracle.tools.bf16_noise_floor
 """
 import torch, math, numpy as np, sys

@@ -3,7 +3,7 @@ UNMODIFIED reference hands to `batch_generate_json` (main.py:305, 412) in steady
 
 bench.py replays them — the reference itself cannot travel to the GPU box.  The game is driven
 through the vllm shim by a scripted backend that answers with schema-valid JSON of the length
-the reference's truncation rules cap at (400-char strategy, 600-char reasoning; SURVEY.md §3.4),
+the reference's truncation rules cap at (400-char strategy, 600-char reasoning),
 always votes "continue" so the game runs to its round limit, and never triggers retries; the
 prompts are therefore exactly what a well-behaved model would make the reference build.
 

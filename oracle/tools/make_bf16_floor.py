@@ -1,7 +1,7 @@
 """ORACLE tool (test infrastructure): what does the reference's OWN model deviate by in bf16?
 
-north_star states "logits within 2e-2 abs in bf16 against an fp32 CPU forward".  That bound holds
-at the 0.6B architecture; at the widths of the other BASELINE configs the random-init logits are
+The requirement is "logits within 2e-2 abs in bf16 against an fp32 CPU forward".  That bound holds
+at the 0.6B architecture; at the widths of the other configurations the random-init logits are
 2-2.5x larger (std 0.02*sqrt(d_model)) and so is every bf16 rounding.  To give the per-width
 tolerances an independent footing this script runs transformers' own model — the oracle's model,
 unchanged code (modeling_qwen3.py / modeling_mistral.py) — twice on the CPU with the SAME

@@ -1,6 +1,6 @@
 """Generates byzantine_consensus_llm_agents_b200/assets/bpe_merges.json.
 
-No tokenizer or model files exist offline (SURVEY.md F9), so the engine ships a deterministic
+No tokenizer or model files exist offline, so the engine ships a deterministic
 synthetic byte-level BPE tokenizer.  Its merges are trained here, once, on the prompts the
 UNMODIFIED reference builds (driven through the vllm shim with a scripted JSON backend), so
 that the reference's prompts tokenise at a realistic ~4 chars/token.  Run from the repo root:

@@ -1,6 +1,5 @@
 #!/usr/bin/env python
-"""Times the sm_100 incumbents the reference reaches through vLLM (SURVEY.md §2.1 "incumbent"
-column) next to this repo's kernels, on the bench's shapes, on the same GPU in the same process:
+"""Times the sm_100 incumbents the reference reaches through vLLM next to this repo's kernels, on the bench's shapes, on the same GPU in the same process:
 
   K3/K9-K12  cuBLAS bf16 (torch.matmul)          vs bcg_gemm_bf16_tn     decode M=10 and prefill M=12,390
   K8         FlashInfer paged decode (trtllm-gen) vs bcg_decode_attn_paged  B=10, S=1600, 40:8 heads
@@ -12,7 +11,7 @@ Timing: CUDA events around a CUDA graph of back-to-back launches over DISTINCT w
 (decode shapes: inputs >> L2), after warm-up.  A section that cannot run here (FlashInfer needs a
 JIT build or a cubin that is not in the image, ...) is recorded as {"unavailable": "<error text>"}.
 
-    python tools/incumbent_kernels.py --out gpurun_out/incumbent_kernels.json
+    python tools/incumbent_kernels.py --out incumbent_kernels.json
 """
 import argparse
 import json
@@ -100,7 +99,7 @@ def section(results, name, limit_s=240):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default="gpurun_out/incumbent_kernels.json")
+    ap.add_argument("--out", default="incumbent_kernels.json")
     ap.add_argument("--skip-flashinfer", action="store_true")
     a = ap.parse_args()
     torch.cuda.set_device(0)

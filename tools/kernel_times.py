@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Per-kernel decode-step timing with CUDA events (dev tool; feeds the roofline table in DESIGN.md).
+"""Per-kernel decode-step timing with CUDA events (dev tool).
 
 Each kernel is launched back to back over all layers' weights / KV (inputs >> L2), so the average
 is a warm-pipeline, cold-data figure — the regime inside the decode CUDA graph.

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""BASELINE.json configs[4]: Qwen3-32B, tensor parallel over the GPUs of one box, agent-count sweep
+"""Qwen3-32B, tensor parallel over the GPUs of one box, agent-count sweep
 N in {4, 8, 16, 32, 64} with floor(0.2 N) Byzantine agents — ONE model load, one JSON line per N
 (dev / evidence tool; bench.py stays the contract-shaped benchmark).
 
