@@ -232,8 +232,8 @@ sandwich_row_kernel(float* residual, const float* delta, int n_partials, long lo
   if (mine && xn) store_vec<4>(xn + t * d + 4 * v, x);
 }
 
-// Prompts: a row per CTA, kept in registers; all reads of a thread are on their way before the first is used.  12,390 rows of 2048:
-// 91 -> 74 us (a row staged in shared memory before), 6,500 with eight experts' rows each 123 -> 103.
+// Prompts: a row per CTA, kept in registers; all reads of a thread are on their way before the first is used.  12,436 rows of 2048:
+// 90 -> 76 us (a row staged in shared memory before), 6,378 with eight experts' rows each 150 -> 129.
 template <typename T, int THREADS, int NV>
 __global__ void __launch_bounds__(THREADS)
 sandwich_long_kernel(float* residual, const float* delta, int n_partials, long long partial_stride, const float* __restrict__ w_post,
@@ -388,7 +388,7 @@ poly_norm_kernel(const float* __restrict__ z, int n_partials, long long partial_
 }
 
 // NV vectors per thread, kept in registers between the sums and the polynomial: a few rows over clusters (eight of 7424 in a captured
-// step: 7.2 -> 5.4 us), or prompts with a CTA per row (12,390 of 7424: 127 -> 106 us).
+// step: 7.2 -> 5.4 us), or prompts with a CTA per row (12,436 of 7424: 125 -> 109 us).
 template <typename T, int NV, int CL>
 __global__ void __launch_bounds__(kRowT)
 poly_row_kernel(const float* z, int n_partials, long long partial_stride, const float* __restrict__ coef, T* out, int ff, float eps) {
