@@ -4,8 +4,8 @@ Two independent things shard with no data-path collective:
   * ROWS of one `batch_generate_json` call — every (agent, phase) generation depends only on its
     own prompt.  All ranks run the same game script (same seeds -> same prompts), each decodes the
     rows `shard_rows()` gives it, and the texts are exchanged host-side (`gather_rows`, an
-    all_gather_object of a few KB).  Per-row results are batch-invariant and seeded by the row's
-    GLOBAL index, so the gathered result equals the single-GPU one.
+    all_gather_object of a few KB).  Per-row results are batch-invariant (layer stacks: but for
+    rounding) and seeded by the row's GLOBAL index, so the gathered result equals the single-GPU one.
   * whole GAMES — one game per replica (bench.py --gpus N, weak scaling).
 Only host objects cross ranks (gloo or NCCL object collectives); device collectives are not used.
 """

@@ -10,8 +10,8 @@ the host only polls a single counter every few steps to stop early.
 Differences from the engine the reference reaches (deliberate):
   * every row of a call is decoded together, each with its own grammar (the reference falls
     back to one-prompt-at-a-time when schemas differ, vllm_agent.py:417-455) and without the
-    `max_num_seqs=4` cap (config.py:38) — per-row results are batch-invariant, so this changes
-    scheduling, not outputs;
+    `max_num_seqs=4` cap (config.py:38) — per-row results are batch-invariant (layer stacks: but for
+    rounding), so this changes scheduling, not outputs;
   * KV pages of a prompt's full 16-token blocks stay cached ACROSS calls and rounds, keyed by a
     hash chain over token ids (same idea as vLLM's enable_prefix_caching): per-agent system
     prompts and identical retry prompts (main.py:293-317) are not prefilled twice.
